@@ -26,7 +26,7 @@ namespace bhcb {
 template<typename R> cudaError_t launch_trace(const GroupDev *, int, long long, void *,
                                               unsigned long long, RunCounters *,
                                               unsigned long long *, unsigned int *, int, int, cudaStream_t,
-                                              unsigned int, int);
+                                              unsigned int, int, int);
 cudaError_t launch_influence_mixed(const void *, unsigned long long, const GroupDev *, int, const double *,
                                    float2 *, RunCounters *, bool, bool, int, cudaStream_t, unsigned int *,
                                    unsigned long long *);
@@ -307,6 +307,37 @@ cudaError_t record_event(bhcb_ctx *c, int k, cudaStream_t st)
                         : cudaEventRecord(c->ev[k], st);
 }
 
+// The profile type shared by groups [g0, g1) if all have packed segments, else
+// 0: a launch runs one step routine, so a batch of several profile types, or
+// one with attenuation in the water, takes the general one.
+int seg_kind(const bhcb_ctx *c, int g0, int g1)
+{
+    const EnvDev &a = c->envdev_h[g0];
+    for(int g = g0; g < g1; ++g)
+        if(!c->envdev_h[g].has_seg || c->envdev_h[g].ssp_type != a.ssp_type) return 0;
+    return a.ssp_type;
+}
+
+// Packed segments of a profile of type C, S or P; empty for other types, for
+// complex sound speeds and for fewer than two nodes.
+std::vector<SspSeg> pack_segments(const EnvTables &T)
+{
+    std::vector<SspSeg> v;
+    const size_t n = T.z.size();
+    const bool lin = T.ssp_type == SSP_CLINEAR;
+    if(n < 2 || (!lin && T.ssp_type != SSP_CUBIC && T.ssp_type != SSP_PCHIP)) return v;
+    auto coef = [&](size_t k, size_t i, int part) {
+        if(lin) return k == 0 ? T.c[2 * i + part] : k == 1 ? T.cz[2 * i + part] : 0.0;
+        return T.coef[2 * (k * n + i) + part];
+    };
+    for(size_t i = 0; i + 1 < n; ++i) {
+        for(size_t k = 0; k < 4; ++k)
+            if(coef(k, i, 1) != 0.0) return {};
+        v.push_back(SspSeg{T.z[i], T.z[i + 1], coef(0, i, 0), coef(1, i, 0), coef(2, i, 0), coef(3, i, 0), {0.0, 0.0}});
+    }
+    return v;
+}
+
 void do_prepare(bhcb_ctx *c)
 {
     if(c->envs.empty()) throw StateError("no environment: call bhcb_setup or bhcb_add_env first");
@@ -367,7 +398,7 @@ void do_prepare(bhcb_ctx *c)
     }
     // --- build device tables
     Arena A;
-    struct EnvOffsets { size_t z, rho, c, cz, n2, n2z, coef, qr, qc, qcz, trc, brc, btop, bbot, rr, rz, sz, alpha, acs, sbp; };
+    struct EnvOffsets { size_t z, rho, c, cz, n2, n2z, coef, seg, qr, qc, qcz, trc, brc, btop, bbot, rr, rz, sz, alpha, acs, sbp; };
     std::vector<EnvOffsets> offs;
     std::vector<EnvDev> envdev;
     for(const GroupPlan &gp : plan) {
@@ -376,6 +407,8 @@ void do_prepare(bhcb_ctx *c)
         EnvOffsets o;
         o.z = A.put(T.z); o.rho = A.put(T.rho); o.c = A.put(T.c); o.cz = A.put(T.cz);
         o.n2 = A.put(T.n2); o.n2z = A.put(T.n2z); o.coef = A.put(T.coef);
+        const std::vector<SspSeg> seg = pack_segments(T);
+        o.seg = A.put(seg);
         o.qr = A.put(T.qr); o.qc = A.put(T.qc); o.qcz = A.put(T.qcz);
         o.trc = A.put(T.trc); o.brc = A.put(T.brc);
         o.btop = A.put(T.btop); o.bbot = A.put(T.bbot);
@@ -393,6 +426,7 @@ void do_prepare(bhcb_ctx *c)
         EnvDev d{};
         d.ssp_type = T.ssp_type;
         d.nssp = (int)T.z.size();
+        d.has_seg = !seg.empty();
         d.nqr = (int)T.qr.size();
         d.ntrc = (int)(T.trc.size() / 3);
         d.nbrc = (int)(T.brc.size() / 3);
@@ -448,6 +482,7 @@ void do_prepare(bhcb_ctx *c)
         d.c = dptr<double>(ab, o.c); d.cz = dptr<double>(ab, o.cz);
         d.n2 = dptr<double>(ab, o.n2); d.n2z = dptr<double>(ab, o.n2z);
         d.coef = dptr<double>(ab, o.coef);
+        d.segtab = dptr<SspSeg>(ab, o.seg);
         d.qr = dptr<double>(ab, o.qr); d.qc = dptr<double>(ab, o.qc); d.qcz = dptr<double>(ab, o.qcz);
         d.trc = dptr<double>(ab, o.trc); d.brc = dptr<double>(ab, o.brc);
         d.btop = dptr<BdryPtDev>(ab, o.btop); d.bbot = dptr<BdryPtDev>(ab, o.bbot);
@@ -591,10 +626,10 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
     }
     if(fp64)
         CK(launch_trace<double>(G, ng, job1, c->segs.p, c->seg_cap, ctr, jobc, blk, (int)tgrid, tblock,
-                                c->stream, stage_bytes, c->trace_lanes));
+                                c->stream, stage_bytes, c->trace_lanes, seg_kind(c, g0, g1)));
     else
         CK(launch_trace<float>(G, ng, job1, c->segs.p, c->seg_cap, ctr, jobc, blk, (int)tgrid, tblock,
-                               c->stream, stage_bytes, c->trace_lanes));
+                               c->stream, stage_bytes, c->trace_lanes, seg_kind(c, g0, g1)));
     CK(record_event(c, 1, c->stream));
     if(c->mode != MODE_TL) return;   // arrivals / hits: run_arrivals after the trace
     if(ovl) {
@@ -706,10 +741,10 @@ void launch_pipelined(bhcb_ctx *c)
     if(tgrid < 1) tgrid = 1;
     if(fp64)
         CK(launch_trace<double>(G, ng, c->njobs, segs, c->seg_cap, ctr, jobc, nullptr, (int)tgrid, tblock, A,
-                                stage_bytes, c->trace_lanes));
+                                stage_bytes, c->trace_lanes, seg_kind(c, 0, ng)));
     else
         CK(launch_trace<float>(G, ng, c->njobs, segs, c->seg_cap, ctr, jobc, nullptr, (int)tgrid, tblock, A,
-                               stage_bytes, c->trace_lanes));
+                               stage_bytes, c->trace_lanes, seg_kind(c, 0, ng)));
     CK(cudaEventRecord(ev[1], A));
     CK(cudaStreamWaitEvent(Bs, ev[1], 0));
     CK(cudaEventRecord(ev[2], Bs));

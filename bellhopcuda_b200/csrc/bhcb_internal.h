@@ -47,6 +47,13 @@ struct BdryPtDev {      // 2-D boundary node (include/bhc/structs.hpp:147-170)
     double cPr, cPi, cSr, cSi, rho;   // per-segment halfspace (long format 'L')
 };
 
+// One interval of a 1-D profile of type C, S or P with a real sound speed: its
+// depth bounds and its coefficients (C: c and dc/dz; S, P: the four of the
+// polynomial in z - z0). One 64-byte record, read by 16-byte loads.
+struct alignas(16) SspSeg {
+    double z0, z1, k0, k1, k2, k3, pad[2];
+};
+
 struct EnvDev {
     // SSP tables (reference SSPStructure, include/bhc/structs.hpp:73-91)
     int32_t ssp_type, nssp;
@@ -54,6 +61,8 @@ struct EnvDev {
     const double *c, *cz;      // complex, interleaved re/im, [nssp]
     const double *n2, *n2z;    // complex [nssp]
     const double *coef;        // complex [4][nssp]: spline (S) or pchip (P) coefficients
+    int32_t has_seg, pad_s;    // segtab holds the profile: type C, S or P, no attenuation
+    const SspSeg *segtab;      // [nssp - 1]
     // quad (range-dependent) SSP (src/ssp.hpp:157-212): profile ranges qr[nqr]
     // (m), sound speed qc[iz * nqr + ir] and its depth gradient qcz[iz * nqr + ir]
     int32_t nqr, pad_q;

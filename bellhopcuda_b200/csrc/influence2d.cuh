@@ -50,60 +50,77 @@ struct InflState {   // the carried part of InfluenceRayInfo (include/bhc/struct
     double phase, qOld;
     V2<double> x;
     int ir;
+    double r;            // the receiver range rr[ir]
+};
+
+// What the prologue reads of the environment, held in registers over a ray.
+struct InflEnv {
+    const double *rr;
+    int nrr, gaussian, arrivals;
+    __device__ __forceinline__ explicit InflEnv(const EnvDev &e)
+        : rr(e.rr), nrr(e.nrr), gaussian(e.gaussian), arrivals(e.arrivals) {}
 };
 
 // Sequential prologue of Step_InfluenceGeoCart (2-D): returns true when the
 // segment has receiver columns to evaluate and fills rec.
 template<typename R, typename RecR> __device__ __forceinline__ bool infl_prologue(
-    const RayPt<R> &p0, const RayPt<R> &p1, InflState &inf, const EnvDev &e, R rcp_q0, R ratio1,
+    const RayPt<R> &p0, const RayPt<R> &p1, InflState &inf, const InflEnv &e, R rcp_q0, R ratio1,
     int job, int is, SegRec<RecR> &rec)
 {
     double rA = inf.x.x, rB = p1.x.x;
     V2<double> d = sub2(p1.x, p0.x);
-    // IsSmallValue(rlen): duplicate point. rlen = |d| is needed only by
-    // segments that reach a receiver column; when |d|^2 exceeds four times the
-    // squared threshold, rlen is above the threshold whatever the rounding,
-    // and the square root waits until the segment is stored.
+    // IsSmallValue(rlen): duplicate point, shorter than 1000 spacings of
+    // doubles at x. rlen = |d| is needed only by segments that reach a receiver
+    // column; when |d| > 1e-12 |x| it is above the threshold (1000 spacings are
+    // at most 2.3e-13 |x|), and the square root waits until the segment is stored.
     const double dd = dot2(d, d);
-    const double small_len = 1.0e3 * spacing_d(p1.x.x);
     double rlen = 0.0;
-    const bool long_seg = dd > 4.0 * small_len * small_len;
+    const bool long_seg = dd > 1.0e-24 * (p1.x.x * p1.x.x) && dd > 1.0e-200;
     if(!long_seg) {
         rlen = sqrt(dd);
-        if(rlen < small_len) return false;
+        if(rlen < 1.0e3 * spacing_d(p1.x.x)) return false;
     }
     double phaseq = (double)p0.q.x;
     if((phaseq <= 0.0 && inf.qOld > 0.0) || (phaseq >= 0.0 && inf.qOld < 0.0))
         inf.phase += BHCB_PI / FLTD(2.0);
     inf.qOld = phaseq;
-    // receiver-column walk (src/influence.hpp:1295-1402 loop control)
+    // receiver-column walk (src/influence.hpp:1295-1402 loop control); the
+    // range of the current column is carried, one table load per column
     double lo = min(rA, rB), hi = max(rA, rB);
     int first = -1, last = -2;
     int ir = inf.ir;
+    double r = inf.r;
     const double *rr = e.rr;
-    for(int guard = 0; guard <= e.nrr; ++guard) {
-        double r = rr[ir];
+    const int nrr = e.nrr;
+    for(int guard = 0; guard <= nrr; ++guard) {
         if(r >= lo && r < hi) {
             if(first < 0) first = ir;
             last = ir;
         }
         int irTT;
+        double rTT;
         if(rB > r) {
-            if(ir >= e.nrr - 1) break;
+            if(ir >= nrr - 1) break;
             irTT = ir + 1;
-            if(rr[irTT] >= rB) break;
+            rTT = rr[irTT];
+            if(rTT >= rB) break;
         } else {
             if(ir <= 0) break;
             irTT = ir - 1;
-            if(rr[irTT] <= rB) break;
+            rTT = rr[irTT];
+            if(rTT <= rB) break;
         }
         ir = irTT;
+        r = rTT;
     }
     inf.ir = ir;
+    inf.r = r;
     inf.x = p1.x;
     if(first < 0) return false;
-    if(long_seg) rlen = sqrt(dd);
-    const V2<double> rayt = div2(d, rlen);
+    if(long_seg) rlen = sqrt_rn(dd);
+    const double rcp_len = rcp_ulp(rlen);
+    const V2<double> rayt = mk2(quot_rn(d.x, rlen, rcp_len), quot_rn(d.y, rlen, rcp_len));
+    const double atx = fabs(rayt.x);
     rec.x0r = p0.x.x;
     rec.x0z = p0.x.y;
     rec.tau0r = p0.taur;
@@ -116,11 +133,14 @@ template<typename R, typename RecR> __device__ __forceinline__ bool infl_prologu
     rec.q0 = (RecR)p0.q.x;
     rec.dq = (RecR)(p1.q.x - p0.q.x);
     rec.rcp_q0 = (RecR)rcp_q0;
-    rec.cnst_num = (RecR)(ratio1 * sqrt(p1.c) * p1.Amp);
+    rec.cnst_num = (RecR)(ratio1 * (sizeof(R) == 8 ? (R)sqrt_rn((double)p1.c) : (R)sqrt(p1.c)) * p1.Amp);
     const RayPt<R> &pp = e.gaussian ? p1 : p0;
     rec.phase_a = (RecR)((double)pp.Phase + inf.phase);
     rec.phase_b = (RecR)(inf.phase + BHCB_PI / FLTD(2.0));
-    rec.sigma_seg = (RecR)(max(fabs(p0.q.x), fabs(p1.q.x)) * rcp_q0 / (R)fabs(rayt.x));
+    // max|q| rcp_q0 / |tx|; a vertical segment (tx 0 or negligible) keeps IEEE division's infinity
+    const R qmax = max(fabs(p0.q.x), fabs(p1.q.x)) * rcp_q0;
+    if(sizeof(R) == 8 && atx > 1.0e-100) rec.sigma_seg = (RecR)div_rn((double)qmax, atx);
+    else rec.sigma_seg = (RecR)(qmax / (R)atx);
     rec.c0 = (RecR)p0.c;
     rec.tau1r = (RecR)p1.taur;
     rec.zlo = (RecR)min(p0.x.y, p1.x.y);

@@ -23,13 +23,16 @@
 #include "trace2d.cuh"
 #include "influence2d.cuh"
 #include "ray2d.cuh"
+#include "ray2seg.cuh"
 #include "tabstage.cuh"
 
 namespace bhcb {
 
-// R: ray state; RecR: segment record (float for the mixed kernel's FP32 influence).
+// R: ray state; RecR: segment record (float for the mixed kernel's FP32
+// influence); K: the profile type when every group of the launch has packed
+// profile segments of that type (ray2seg.cuh), else 0.
 // lanes: rays per warp (16 or 32); the other lanes only help stage the tables.
-template<typename R, typename RecR> __global__ void __launch_bounds__(64) trace_kernel(
+template<typename R, typename RecR, int K> __global__ void __launch_bounds__(64) trace_kernel(
     const GroupDev *__restrict__ groups, int ngroups, long long njobs, SegRec<RecR> *segs,
     unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, unsigned int *blk_state,
     unsigned int stage_budget, int lanes)
@@ -58,11 +61,8 @@ template<typename R, typename RecR> __global__ void __launch_bounds__(64) trace_
         // ---- RayInit (src/trace.hpp:76-266)
         RayState2<R> st;
         if(!ray_init2d(e, ialpha, isz, st, ctr)) continue;
-        RayPt<R> &p0 = st.p0;
-        RayPt<R> p1, p2;
         const double alpha = st.alpha;
         const R c = st.c;
-        double dEndTop, dEndBot;
         // ---- Init_Influence (src/influence.hpp:525-644), Cartesian geometric
         R ratio1 = (R)sqrt(fabs(cos(alpha)));
         if(e.line_source) ratio1 = (R)1;
@@ -70,31 +70,49 @@ template<typename R, typename RecR> __global__ void __launch_bounds__(64) trace_
         R rcp_q0 = (R)(e.dalpha / (double)c);
         InflState inf;
         inf.phase = 0.0;
-        inf.qOld = (double)p0.q.x;
-        inf.x = p0.x;
-        inf.ir = bsearch_gt(e.rr, e.nrr, p0.x.x);
-        if(p0.t.x < (R)0 && inf.ir > 0) --inf.ir;
+        inf.qOld = (double)st.p0.q.x;
+        inf.x = st.p0.x;
+        inf.ir = bsearch_gt(e.rr, e.nrr, st.p0.x.x);
+        if(st.p0.t.x < (R)0 && inf.ir > 0) --inf.ir;
+        inf.r = e.rr[inf.ir];
 
+        const InflEnv ie(e);
         int small = 0, is = 0;
+        double dEndTop = 0.0, dEndBot = 0.0;
         bool overflow = false;
-        unsigned long long nsteps = 0;
+        unsigned int nsteps = 0;
         SlotCursor cur;
+        auto influence = [&](const RayPt<R> &a, const RayPt<R> &b) {
+            SegRec<RecR> rec;
+            if(infl_prologue(a, b, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
+                emit_seg(rec, segs, cap, ctr, cur, overflow, blk_state);
+            ++is;
+        };
+        Ray2Seg<K> ray;
+        if constexpr(K != 0) ray.init(st, e);
+        RayPt<R> p1, p2;
         for(;;) {
             // another ray's error stops the run (src/trace.hpp:559); polled every 32 steps
             if((nsteps & 31) == 0 && __ldcg(&ctr->err_bits) != 0u) break;
-            const bool two = ray_update2d(st, p1, p2, small, dEndTop, dEndBot, e, ctr);
             ++nsteps;
-            SegRec<RecR> rec;
-            if(infl_prologue(p0, p1, inf, e, rcp_q0, ratio1, (int)job, is, rec))
-                emit_seg(rec, segs, cap, ctr, cur, overflow, blk_state);
-            ++is;
-            if(two) {
-                if(infl_prologue(p1, p2, inf, e, rcp_q0, ratio1, (int)job, is, rec))
-                    emit_seg(rec, segs, cap, ctr, cur, overflow, blk_state);
-                p0 = p2;
-                ++is;
+            if constexpr(K != 0) {
+                const int hit = ray.step(p1, ctr);
+                influence(ray.p0, p1);
+                ray.p0 = p1;
+                if(hit) {
+                    ray.reflect(hit, ctr);
+                    // the segment to the reflected point has no length, which leaves
+                    // the influence state as it is, unless the point was displaced
+                    // or lies at range 0 (where the threshold of length is 0)
+                    p2 = ray.p0;
+                    if(!(p2.x.x == p1.x.x && p2.x.y == p1.x.y && p1.x.x != 0.0)) influence(p1, p2);
+                    else ++is;
+                }
             } else {
-                p0 = p1;
+                const bool two = ray_update2d(st, p1, p2, small, dEndTop, dEndBot, e, ctr);
+                influence(st.p0, p1);
+                if(two) influence(p1, p2);
+                st.p0 = two ? p2 : p1;
             }
             if(overflow) {
                 atomicMin(&ctr->overflow_job, (unsigned int)job);
@@ -102,16 +120,20 @@ template<typename R, typename RecR> __global__ void __launch_bounds__(64) trace_
                 break;
             }
             // ---- RayTerminate (src/trace.hpp:391-477), 2-D
-            if(ray_stops2d(st, dEndTop, dEndBot, e)) break;
+            if constexpr(K != 0) {
+                if(ray.stops()) break;
+            } else {
+                if(ray_stops2d(st, dEndTop, dEndBot, e)) break;
+                st.dBegTop = dEndTop;
+                st.dBegBot = dEndBot;
+            }
             if(is >= MAXN_STEPS - 3) {
                 run_warn(ctr, WARN_ONERAY_OUTOFMEMORY);
                 break;
             }
-            st.dBegTop = dEndTop;
-            st.dBegBot = dEndBot;
         }
         close_block(segs, cur, blk_state);
-        atomicAdd(&ctr->nsteps, nsteps);
+        atomicAdd(&ctr->nsteps, (unsigned long long)nsteps);
     }
     if(stage_budget > 0 && !staged) stage_drain(&s_bar);
 }
@@ -478,26 +500,43 @@ cudaError_t launch_set_counter(unsigned long long *p, unsigned long long v, cuda
     return cudaGetLastError();
 }
 
-template<typename R> cudaError_t launch_trace(const GroupDev *groups, int ngroups, long long njobs,
-                                              void *segs, unsigned long long cap, RunCounters *ctr,
-                                              unsigned long long *job_counter, unsigned int *blk_state,
-                                              int grid, int block, cudaStream_t st, unsigned int stage_bytes,
-                                              int lanes)
+namespace {
+template<typename R, int K> cudaError_t launch_trace_k(const GroupDev *groups, int ngroups, long long njobs, void *segs,
+                                                       unsigned long long cap, RunCounters *ctr,
+                                                       unsigned long long *job_counter, unsigned int *blk_state,
+                                                       int grid, int block, cudaStream_t st,
+                                                       unsigned int stage_bytes, int lanes)
 {
     // the ray state is FP64 in both precisions (the mixed precision writes FP32
     // segment records for its FP32 influence kernel): the trajectory, and with it
     // every step and reflection decision, is the FP64 one
     static bool attr_set = false;
     if(!attr_set) {   // dynamic shared memory above the 48 KB default
-        cudaError_t e = cudaFuncSetAttribute(trace_kernel<double, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(trace_kernel<double, R, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)STAGE_MAX_BYTES);
         if(e != cudaSuccess) return e;
         attr_set = true;
     }
     if(stage_bytes > STAGE_MAX_BYTES) stage_bytes = STAGE_MAX_BYTES;
-    trace_kernel<double, R><<<grid, block, stage_bytes, st>>>(groups, ngroups, njobs, (SegRec<R> *)segs, cap, ctr,
-                                                              job_counter, blk_state, stage_bytes, lanes);
+    trace_kernel<double, R, K><<<grid, block, stage_bytes, st>>>(groups, ngroups, njobs, (SegRec<R> *)segs, cap, ctr,
+                                                                 job_counter, blk_state, stage_bytes, lanes);
     return cudaGetLastError();
+}
+} // namespace
+
+// kind: the profile type of every launched group when all have packed segments
+// (SSP_CLINEAR, SSP_CUBIC, SSP_PCHIP), else 0
+template<typename R> cudaError_t launch_trace(const GroupDev *groups, int ngroups, long long njobs,
+                                              void *segs, unsigned long long cap, RunCounters *ctr,
+                                              unsigned long long *job_counter, unsigned int *blk_state,
+                                              int grid, int block, cudaStream_t st, unsigned int stage_bytes,
+                                              int lanes, int kind)
+{
+    auto f = launch_trace_k<R, 0>;
+    if(kind == SSP_CLINEAR) f = launch_trace_k<R, SSP_CLINEAR>;
+    else if(kind == SSP_CUBIC) f = launch_trace_k<R, SSP_CUBIC>;
+    else if(kind == SSP_PCHIP) f = launch_trace_k<R, SSP_PCHIP>;
+    return f(groups, ngroups, njobs, segs, cap, ctr, job_counter, blk_state, grid, block, st, stage_bytes, lanes);
 }
 
 cudaError_t launch_influence_mixed(const void *segs, unsigned long long cap, const GroupDev *groups, int ngroups,
@@ -539,10 +578,10 @@ cudaError_t launch_scale(const float2 *acc, float2 *out, const GroupDev *groups,
 
 template cudaError_t launch_trace<float>(const GroupDev *, int, long long, void *, unsigned long long,
                                          RunCounters *, unsigned long long *, unsigned int *, int, int,
-                                         cudaStream_t, unsigned int, int);
+                                         cudaStream_t, unsigned int, int, int);
 template cudaError_t launch_trace<double>(const GroupDev *, int, long long, void *, unsigned long long,
                                           RunCounters *, unsigned long long *, unsigned int *, int, int,
-                                          cudaStream_t, unsigned int, int);
+                                          cudaStream_t, unsigned int, int, int);
 template cudaError_t launch_influence<float>(const void *, unsigned long long, const GroupDev *, int,
                                              const double *, float2 *, RunCounters *, bool, bool, int,
                                              cudaStream_t);

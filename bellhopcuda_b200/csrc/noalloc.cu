@@ -198,12 +198,14 @@ noalloc_trace_kernel(unsigned char *scratch, double freq)
         if(e.line_source) ratio1 = (R)1;
         if(e.gaussian) ratio1 = (R)((double)ratio1 / sqrt(FLTD(2.0) * BHCB_PI));
         R rcp_q0 = (R)(e.dalpha / (double)c);
+        const InflEnv ie(e);
         InflState inf;
         inf.phase = 0.0;
         inf.qOld = (double)p0.q.x;
         inf.x = p0.x;
         inf.ir = bsearch_gt(e.rr, e.nrr, p0.x.x);
         if(p0.t.x < (R)0 && inf.ir > 0) --inf.ir;
+        inf.r = e.rr[inf.ir];
         int small = 0, is = 0;
         unsigned long long nsteps = 0;
         for(;;) {
@@ -235,11 +237,11 @@ noalloc_trace_kernel(unsigned char *scratch, double freq)
                 distances(p2.x, top, bot, dEndTop, dEndBot);
             }
             SegRec<RecR> rec;
-            if(infl_prologue(p0, p1, inf, e, rcp_q0, ratio1, (int)job, is, rec))
+            if(infl_prologue(p0, p1, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
                 eval_segment_inline<RecR, GAUSS, COHERENT>(rec, e, freq, acc, base, evals);
             ++is;
             if(two) {
-                if(infl_prologue(p1, p2, inf, e, rcp_q0, ratio1, (int)job, is, rec))
+                if(infl_prologue(p1, p2, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
                     eval_segment_inline<RecR, GAUSS, COHERENT>(rec, e, freq, acc, base, evals);
                 p0 = p2;
                 ++is;

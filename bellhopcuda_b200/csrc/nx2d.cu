@@ -383,12 +383,14 @@ __global__ void __launch_bounds__(64) trace_nx_kernel(const GroupDev *__restrict
         double ratio1 = sqrt(fabs(cos(st.alpha)));
         if(e.gaussian) ratio1 /= sqrt(FLTD(2.0) * BHCB_PI);
         const double rcp_q0 = E.dalpha / st.c;
+        const InflEnv ie(e);
         InflState inf;
         inf.phase = 0.0;
         inf.qOld = p0.q.x;
         inf.x = p0.x;
         inf.ir = bsearch_gt(e.rr, e.nrr, p0.x.x);
         if(p0.t.x < 0.0 && inf.ir > 0) --inf.ir;
+        inf.r = e.rr[inf.ir];
         int small = 0, is = 0;
         bool overflow = false;
         unsigned long long nsteps = 0;
@@ -398,11 +400,11 @@ __global__ void __launch_bounds__(64) trace_nx_kernel(const GroupDev *__restrict
             const bool two = ray_update_nx(st, p1, p2, small, E, ctr);
             ++nsteps;
             SegRec<double> rec;
-            if(infl_prologue(p0, p1, inf, e, rcp_q0, ratio1, (int)job, is, rec))
+            if(infl_prologue(p0, p1, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
                 emit_nx(rec, segs, cap, ctr, cur, overflow);
             ++is;
             if(two) {
-                if(infl_prologue(p1, p2, inf, e, rcp_q0, ratio1, (int)job, is, rec))
+                if(infl_prologue(p1, p2, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
                     emit_nx(rec, segs, cap, ctr, cur, overflow);
                 p0 = p2;
                 ++is;

@@ -21,8 +21,9 @@
 namespace bhcb {
 
 // in the order of their reads per step: SSP nodes and coefficients (three
-// evaluations per step), boundary nodes (segment checks), receiver ranges
-enum StageTable : int { ST_Z, ST_C, ST_CZ, ST_COEF, ST_N2, ST_N2Z, ST_RHO, ST_QR, ST_QC, ST_QCZ, ST_BTOP, ST_BBOT,
+// evaluations per step; the packed segments in their place where there are
+// any), boundary nodes (segment checks), receiver ranges
+enum StageTable : int { ST_SEG, ST_Z, ST_C, ST_CZ, ST_COEF, ST_N2, ST_N2Z, ST_RHO, ST_QR, ST_QC, ST_QCZ, ST_BTOP, ST_BBOT,
                         ST_RR, ST_COUNT };
 
 __host__ __device__ inline size_t round16(size_t b) { return (b + 15) & ~size_t(15); }
@@ -37,15 +38,18 @@ __host__ __device__ inline void stage_table_bytes(const EnvDev &e, size_t b[ST_C
     for(int k = 0; k < ST_COUNT; ++k) b[k] = 0;
     const size_t n = (size_t)e.nssp;
     const int t = e.ssp_type;
-    if(t != SSP_ANALYTIC) {
+    if(e.has_seg) {
+        // the step reads the packed segments; nodes and coefficients only at reflections
+        b[ST_SEG] = (n - 1) * sizeof(SspSeg);
+    } else if(t != SSP_ANALYTIC) {
         b[ST_Z] = n * 8;
         b[ST_RHO] = n * 8;   // reflections (and N2-linear) interpolate the density
     }
-    if(t == SSP_CLINEAR || t == SSP_QUAD) {
+    if((t == SSP_CLINEAR && !e.has_seg) || t == SSP_QUAD) {
         b[ST_C] = 2 * n * 8;
         if(t == SSP_CLINEAR) b[ST_CZ] = 2 * n * 8;
     }
-    if(t == SSP_CUBIC || t == SSP_PCHIP) b[ST_COEF] = 8 * n * 8;
+    if((t == SSP_CUBIC || t == SSP_PCHIP) && !e.has_seg) b[ST_COEF] = 8 * n * 8;
     if(t == SSP_N2LINEAR) {
         b[ST_N2] = 2 * n * 8;
         b[ST_N2Z] = 2 * n * 8;
@@ -124,13 +128,14 @@ __device__ __forceinline__ bool stage_env_tables(const EnvDev *src, EnvDev &s_en
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(s_bar)),
                      "r"((uint32_t)total)
                      : "memory");
-        const void *srcs[ST_COUNT] = {s_env.z, s_env.c, s_env.cz, s_env.coef, s_env.n2, s_env.n2z, s_env.rho,
+        const void *srcs[ST_COUNT] = {s_env.segtab, s_env.z, s_env.c, s_env.cz, s_env.coef, s_env.n2, s_env.n2z, s_env.rho,
                                       s_env.qr, s_env.qc, s_env.qcz, s_env.btop, s_env.bbot, s_env.rr};
         for(int k = 0; k < ST_COUNT; ++k) {
             if(off[k] == (size_t)-1) continue;
             bulk_g2s(s_tab + off[k], srcs[k], (uint32_t)round16(b[k]), s_bar);
         }
         auto at = [&](int k) -> const void * { return off[k] == (size_t)-1 ? nullptr : s_tab + off[k]; };
+        if(at(ST_SEG)) s_env.segtab = (const SspSeg *)at(ST_SEG);
         if(at(ST_Z)) s_env.z = (const double *)at(ST_Z);
         if(at(ST_C)) s_env.c = (const double *)at(ST_C);
         if(at(ST_CZ)) s_env.cz = (const double *)at(ST_CZ);

@@ -568,10 +568,11 @@ template<typename R> __device__ __forceinline__ void beam_shift2d(const RayPt<R>
     np.q = add2(np.q, scl2(sdd * rdd * si * c, old.p));
 }
 
-// src/reflect.hpp:125-452 (2-D branch)
-template<typename R> __device__ __forceinline__ void reflect2d(
-    const RayPt<R> &old, RayPt<R> &np, const HsDev &hs, bool istop, V2<R> tB, V2<R> nB, R kappa,
-    const EnvDev &e, SegState &iSeg, RunCounters *ctr)
+// src/reflect.hpp:125-452 (2-D branch), the profile o (with its density) at
+// the reflection point
+template<typename R> __device__ __forceinline__ void reflect2d_at(
+    const SSPOut<R> &o, const RayPt<R> &old, RayPt<R> &np, const HsDev &hs, bool istop, V2<R> tB, V2<R> nB, R kappa,
+    const EnvDev &e, RunCounters *ctr)
 {
     R Th = dot2(old.t, nB);
     R Tg = dot2(old.t, tB);
@@ -579,8 +580,6 @@ template<typename R> __device__ __forceinline__ void reflect2d(
     np.nbot = old.nbot + (istop ? 0 : 1);
     np.x = old.x;
     np.t = sub2(old.t, scl2((R)2 * Th, nB));
-    SSPOut<R> o;
-    eval_ssp<R, true>(old.x, old.t, o, e, iSeg, ctr);
     R c = o.c;
     np.c = c;
     np.taur = old.taur;
@@ -654,6 +653,15 @@ template<typename R> __device__ __forceinline__ void reflect2d(
         np.Amp = (R)NAN;
         np.Phase = (R)NAN;
     }
+}
+
+template<typename R> __device__ __forceinline__ void reflect2d(
+    const RayPt<R> &old, RayPt<R> &np, const HsDev &hs, bool istop, V2<R> tB, V2<R> nB, R kappa,
+    const EnvDev &e, SegState &iSeg, RunCounters *ctr)
+{
+    SSPOut<R> o;
+    eval_ssp<R, true>(old.x, old.t, o, e, iSeg, ctr);
+    reflect2d_at(o, old, np, hs, istop, tB, nB, kappa, e, ctr);
 }
 
 } // namespace bhcb
