@@ -23,10 +23,10 @@
 #include "tabstage.cuh"
 
 namespace bhcb {
-template<typename R> cudaError_t launch_trace(const GroupDev *, int, long long, void *,
+template<typename R> cudaError_t launch_trace(const GroupDev *, int, int, void *,
                                               unsigned long long, RunCounters *,
                                               unsigned long long *, unsigned int *, int, int, cudaStream_t,
-                                              unsigned int, int, int);
+                                              unsigned int, int);
 cudaError_t launch_influence_mixed(const void *, unsigned long long, const GroupDev *, int, const double *,
                                    float2 *, RunCounters *, bool, bool, int, cudaStream_t, unsigned int *,
                                    unsigned long long *);
@@ -160,7 +160,9 @@ struct bhcb_ctx {
     // launch shapes (bhcb_autotune picks them by timing the prepared workload)
     int trace_block = 32;           // threads per trace CTA (one ray each)
     int influence_ctas_per_sm = 8;  // persistent influence CTAs per SM
-    int trace_lanes = 32;           // rays per trace warp
+    int trace_lanes = 32;           // most rays per trace warp
+    std::vector<double> est_steps;  // per group: expected steps of its longest ray (relative)
+    int nblocks = 0;                // blocks of rays (GroupDev::blk_base)
 
     std::vector<EnvSlot> envs;
     bool prepared = false;
@@ -318,6 +320,72 @@ int seg_kind(const bhcb_ctx *c, int g0, int g1)
     return a.ssp_type;
 }
 
+// Steps of a group's longest rays, up to a factor: a step ends after deltas or
+// at the next profile node, and rays that turn in a duct cross about as many
+// nodes as node spacings fit into the range.
+double expected_steps(const EnvTables &T)
+{
+    const size_t n = T.z.size();
+    const double dz = n > 1 ? (T.z[n - 1] - T.z[0]) / (double)(n - 1) : 0.0;
+    const double est = T.box_x * (1.0 / std::max(T.deltas, 1e-9) + (dz > 0.0 ? 1.0 / dz : 0.0));
+    return std::isfinite(est) && est > 1.0 ? est : 1.0;
+}
+
+// Rays per warp of every group. A ray's step costs a warp more the more rays
+// step with it, since they part at profile nodes, boundaries and receiver
+// columns: per step, 1 ray 1.33 us, 4 rays 1.77, 16 rays 2.5, 32 rays 3.1 (201
+// rays of a Munk channel, longest ray 855 steps). Fewer rays make more warps,
+// and an SM steps about 6 warps before they slow one another (most for
+// instruction fetch: of 20001 rays, 32 per warp take 6.5 ms, 16 per warp 8.2;
+// of 2001, 2 per warp 1.5, 4 per warp 1.75). So: the shortest time T for which
+// every group has a count whose longest ray ends within T, and all groups'
+// warps together fit into T; groups with short rays get full warps, those with
+// the longest rays thin ones. Against 32 rays per warp throughout: 201 rays
+// 2.6 -> 1.2 ms, 2001 rays 2.1 -> 1.55, 7001 rays (range dependent) 6.6 -> 5.9,
+// 24 uneven environments, begun longest first, 72 -> 53; 20001 rays unchanged.
+void plan_lanes(bhcb_ctx *c)
+{
+    static const int L[6] = {1, 2, 4, 8, 16, 32};
+    static const double cost[6] = {1.0, 1.15, 1.33, 1.6, 1.9, 2.35};
+    const size_t ng = c->groups_h.size();
+    const double room = 6.0 * c->sm_count;   // warps in flight
+    int kmax = 5;
+    while(kmax > 0 && L[kmax] > c->trace_lanes) --kmax;
+    auto pick = [&](double est, double t) {
+        int k = kmax;
+        while(k > 0 && est * cost[k] > t) --k;
+        return k;
+    };
+    auto fits = [&](double t) {
+        double sum = 0.0;
+        for(size_t g = 0; g < ng; ++g) {
+            const int k = pick(c->est_steps[g], t);
+            if(c->est_steps[g] * cost[k] > t) return false;
+            sum += std::ceil((double)c->groups_h[g].njobs / L[k]) * c->est_steps[g] * cost[k];
+        }
+        return sum <= room * t;
+    };
+    double hi = 0.0;
+    for(size_t g = 0; g < ng; ++g) hi = std::max(hi, c->est_steps[g] * cost[kmax]);
+    double t = hi;
+    if(fits(hi)) {
+        double lo = 0.0;
+        for(int i = 0; i < 24; ++i) {
+            const double m = 0.5 * (lo + t);
+            if(fits(m)) t = m; else lo = m;
+        }
+    }   // else: more rays than fit at once, full warps throughout
+    c->nblocks = 0;
+    for(size_t g = 0; g < ng; ++g) {
+        GroupDev &G = c->groups_h[g];
+        G.lanes = L[pick(c->est_steps[g], t)];
+        G.blk_base = c->nblocks;
+        c->nblocks += (G.njobs + G.lanes - 1) / G.lanes;
+    }
+    c->groups_d.ensure(ng * sizeof(GroupDev));
+    CK(cudaMemcpyAsync(c->groups_d.p, c->groups_h.data(), ng * sizeof(GroupDev), cudaMemcpyHostToDevice, c->stream));
+}
+
 // Packed segments of a profile of type C, S or P; empty for other types, for
 // complex sound speeds and for fewer than two nodes.
 std::vector<SspSeg> pack_segments(const EnvTables &T)
@@ -396,6 +464,15 @@ void do_prepare(bhcb_ctx *c)
         if((T0.beam_type[0] == 'B') != c->gauss || (T0.run_type[0] == 'C') != c->coherent)
             throw std::runtime_error("a batch must use one beam type and one coherence mode");
     }
+    // longest rays first: the trace kernel takes the groups in order, and a long
+    // ray begun late would end the launch alone (24 uneven environments whose
+    // longest rays take 119 to 17069 steps: profiles with many nodes per depth
+    // and range are the long ones)
+    std::stable_sort(plan.begin(), plan.end(), [&](const GroupPlan &a, const GroupPlan &b) {
+        return expected_steps(c->envs[a.env].tables[a.ifreqs[0]]) > expected_steps(c->envs[b.env].tables[b.ifreqs[0]]);
+    });
+    c->est_steps.clear();
+    for(const GroupPlan &gp : plan) c->est_steps.push_back(expected_steps(c->envs[gp.env].tables[gp.ifreqs[0]]));
     // --- build device tables
     Arena A;
     struct EnvOffsets { size_t z, rho, c, cz, n2, n2z, coef, seg, qr, qc, qcz, trc, brc, btop, bbot, rr, rz, sz, alpha, acs, sbp; };
@@ -524,9 +601,7 @@ void do_prepare(bhcb_ctx *c)
         c->njobs += G.njobs;
         c->groups_h.push_back(G);
     }
-    c->groups_d.ensure(c->groups_h.size() * sizeof(GroupDev));
-    CK(cudaMemcpyAsync(c->groups_d.p, c->groups_h.data(), c->groups_h.size() * sizeof(GroupDev),
-                       cudaMemcpyHostToDevice, c->stream));
+    plan_lanes(c);
     c->stats.h2d_bytes += c->groups_h.size() * sizeof(GroupDev) + c->freqs_h.size() * sizeof(double);
     c->freqs_d.ensure(c->freqs_h.size() * sizeof(double));
     CK(cudaMemcpyAsync(c->freqs_d.p, c->freqs_h.data(), c->freqs_h.size() * sizeof(double),
@@ -570,7 +645,9 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
     RunCounters *ctr = (RunCounters *)c->counters.p;
     CK(cudaMemsetAsync(&ctr->overflow_job, 0xff, sizeof(ctr->overflow_job), c->stream));
     unsigned long long *jobc = (unsigned long long *)((uint8_t *)c->counters.p + sizeof(RunCounters));
-    if(job0) CK(launch_set_counter(jobc, (unsigned long long)job0, c->stream));
+    // the x kinds' trace counts rays, the Cartesian one blocks of rays
+    const long long first = c->xkind ? job0 : (long long)c->groups_h[g0].blk_base;
+    if(first) CK(launch_set_counter(jobc, (unsigned long long)first, c->stream));
     if(clear) {
         const int64_t a0 = c->groups_h[g0].acc_base;
         const int64_t a1 = g1 < ngall ? c->groups_h[g1].acc_base : c->total_acc;
@@ -598,16 +675,15 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
         CK(record_event(c, 3, c->stream));
         return;
     }
+    const int blk0 = c->groups_h[g0].blk_base, blk1 = g1 < ngall ? c->groups_h[g1].blk_base : c->nblocks;
     int tblock = c->trace_block;
     unsigned int stage_bytes = 0;   // tables of the launched groups that fit the staging budget
     for(int g = g0; g < g1; ++g) {
         size_t off[ST_COUNT];
         stage_bytes = std::max<unsigned int>(stage_bytes, (unsigned int)stage_plan(c->envdev_h[g], c->stage_cap, off));
     }
-    // rays per CTA: trace_lanes of each warp's 32 lanes take rays
-    const long long rays_per_cta = std::max(1, tblock * c->trace_lanes / 32);
-    long long tgrid = std::min<long long>((job1 - job0 + rays_per_cta - 1) / rays_per_cta, (long long)c->sm_count * 32);
-    if(tgrid < 1) tgrid = 1;
+    const int warps = tblock / 32;
+    const int tgrid = std::max(1, std::min((blk1 - blk0 + warps - 1) / warps, c->sm_count * 32));
     const GroupDev *G = (const GroupDev *)c->groups_d.p + g0;
     int ng = g1 - g0;
     // mixed TL runs driven by the host: influence kernels on stream2 take the
@@ -625,11 +701,11 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
         CK(record_event(c, 0, c->stream));
     }
     if(fp64)
-        CK(launch_trace<double>(G, ng, job1, c->segs.p, c->seg_cap, ctr, jobc, blk, (int)tgrid, tblock,
-                                c->stream, stage_bytes, c->trace_lanes, seg_kind(c, g0, g1)));
+        CK(launch_trace<double>(G, ng, blk1, c->segs.p, c->seg_cap, ctr, jobc, blk, tgrid, tblock,
+                                c->stream, stage_bytes, seg_kind(c, g0, g1)));
     else
-        CK(launch_trace<float>(G, ng, job1, c->segs.p, c->seg_cap, ctr, jobc, blk, (int)tgrid, tblock,
-                               c->stream, stage_bytes, c->trace_lanes, seg_kind(c, g0, g1)));
+        CK(launch_trace<float>(G, ng, blk1, c->segs.p, c->seg_cap, ctr, jobc, blk, tgrid, tblock,
+                               c->stream, stage_bytes, seg_kind(c, g0, g1)));
     CK(record_event(c, 1, c->stream));
     if(c->mode != MODE_TL) return;   // arrivals / hits: run_arrivals after the trace
     if(ovl) {
@@ -736,15 +812,14 @@ void launch_pipelined(bhcb_ctx *c)
         size_t off[ST_COUNT];
         stage_bytes = std::max<unsigned int>(stage_bytes, (unsigned int)stage_plan(c->envdev_h[g], c->stage_cap, off));
     }
-    const long long rays_per_cta = std::max(1, tblock * c->trace_lanes / 32);
-    long long tgrid = std::min<long long>((c->njobs + rays_per_cta - 1) / rays_per_cta, (long long)c->sm_count * 32);
-    if(tgrid < 1) tgrid = 1;
+    const int warps = tblock / 32;
+    const int tgrid = std::max(1, std::min((c->nblocks + warps - 1) / warps, c->sm_count * 32));
     if(fp64)
-        CK(launch_trace<double>(G, ng, c->njobs, segs, c->seg_cap, ctr, jobc, nullptr, (int)tgrid, tblock, A,
-                                stage_bytes, c->trace_lanes, seg_kind(c, 0, ng)));
+        CK(launch_trace<double>(G, ng, c->nblocks, segs, c->seg_cap, ctr, jobc, nullptr, tgrid, tblock, A,
+                                stage_bytes, seg_kind(c, 0, ng)));
     else
-        CK(launch_trace<float>(G, ng, c->njobs, segs, c->seg_cap, ctr, jobc, nullptr, (int)tgrid, tblock, A,
-                               stage_bytes, c->trace_lanes, seg_kind(c, 0, ng)));
+        CK(launch_trace<float>(G, ng, c->nblocks, segs, c->seg_cap, ctr, jobc, nullptr, tgrid, tblock, A,
+                               stage_bytes, seg_kind(c, 0, ng)));
     CK(cudaEventRecord(ev[1], A));
     CK(cudaStreamWaitEvent(Bs, ev[1], 0));
     CK(cudaEventRecord(ev[2], Bs));
@@ -1946,12 +2021,14 @@ int bhcb_autotune(bhcb_ctx *c, int32_t repeats, bhcb_tuning *out)
         }
         c->trace_block = t.trace_block;
         t.trace_lanes = c->trace_lanes;
-        for(int ln : {16, 32}) {   // rays per trace warp: 16 diverge less, if the warps fit
+        for(int ln : {16, 32}) {   // most rays per trace warp
             c->trace_lanes = ln;
+            plan_lanes(c);
             timed(tr, inf);
             if(tr < t.trace_ms) { t.trace_ms = tr; t.trace_lanes = ln; }
         }
         c->trace_lanes = t.trace_lanes;
+        plan_lanes(c);
         t.stage_kb = (int32_t)(c->stage_cap / 1024);
         for(int kb : {0, 32, 64}) {   // shared-memory table staging
             c->stage_cap = (unsigned int)kb * 1024u;
@@ -1995,6 +2072,7 @@ int bhcb_set_tuning(bhcb_ctx *c, const bhcb_tuning *t)
         c->stage_cap = (unsigned int)t->stage_kb * 1024u;
         c->trace_lanes = t->trace_lanes ? t->trace_lanes : 32;
         drop_graph(c);
+        if(c->prepared) plan_lanes(c);
         return BHCB_OK;
     });
 }

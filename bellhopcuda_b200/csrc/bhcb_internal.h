@@ -167,6 +167,9 @@ struct GroupDev {
     int32_t acc_nz;
     int32_t field_index;     // index of the group's first field in the launch
     const Env3Dev *env3;     // 3-D groups: the environment (env is then null)
+    // 2-D traces: the group's rays in blocks of `lanes` consecutive jobs, one
+    // block per warp; blocks are numbered group after group from blk_base
+    int32_t lanes, blk_base;
 };
 
 // One influence segment (point0 -> point1 of Step_InfluenceGeoCart,

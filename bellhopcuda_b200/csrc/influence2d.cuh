@@ -19,6 +19,17 @@ __device__ __forceinline__ int find_group(const GroupDev *groups, int ngroups, i
     return lo;
 }
 
+// the group of a block of rays
+__device__ __forceinline__ int find_block_group(const GroupDev *groups, int ngroups, int blk)
+{
+    int lo = 0, hi = ngroups - 1;
+    while(lo < hi) {
+        int m = (lo + hi + 1) >> 1;
+        if(groups[m].blk_base <= blk) lo = m; else hi = m - 1;
+    }
+    return lo;
+}
+
 // src/common_run.hpp:61-84 (BinarySearchLEQ) on the pattern table
 __device__ __forceinline__ int bsearch_leq2(const double *a, int n, double t)
 {

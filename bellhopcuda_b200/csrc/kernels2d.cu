@@ -31,28 +31,33 @@ namespace bhcb {
 // R: ray state; RecR: segment record (float for the mixed kernel's FP32
 // influence); K: the profile type when every group of the launch has packed
 // profile segments of that type (ray2seg.cuh), else 0.
-// lanes: rays per warp (16 or 32); the other lanes only help stage the tables.
+// Warps take blocks of rays (GroupDev::lanes consecutive jobs of a group) up to
+// block end_block; how many rays a warp takes is the host's choice (plan_lanes).
 template<typename R, typename RecR, int K> __global__ void __launch_bounds__(64) trace_kernel(
-    const GroupDev *__restrict__ groups, int ngroups, long long njobs, SegRec<RecR> *segs,
-    unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, unsigned int *blk_state,
-    unsigned int stage_budget, int lanes)
+    const GroupDev *__restrict__ groups, int ngroups, int end_block, SegRec<RecR> *segs,
+    unsigned long long cap, RunCounters *ctr, unsigned long long *block_counter, unsigned int *blk_state,
+    unsigned int stage_budget)
 {
     // tables of the group this CTA's first rays belong to, staged in shared memory
     extern __shared__ __align__(16) unsigned char s_tab[];
     __shared__ EnvDev s_env;
     __shared__ __align__(8) uint64_t s_bar;
-    const long long hint = min(njobs - 1, groups[0].job_base + (long long)blockIdx.x * blockDim.x);
-    const int gs = find_group(groups, ngroups, hint);
+    const int lane = (int)(threadIdx.x & 31);
+    const int hint = min(end_block - 1, groups[0].blk_base + (int)(blockIdx.x * (blockDim.x >> 5)));
+    const int gs = find_block_group(groups, ngroups, hint);
     const bool staged = stage_budget > 0 && stage_env_tables(groups[gs].env, s_env, s_tab, stage_budget, &s_bar, ctr);
     for(;;) {
-        // a warp with fewer rays takes fewer divergent paths per step
-        if((int)(threadIdx.x & 31) >= lanes) break;
-        long long job = (long long)atomicAdd(job_counter, 1ull);
-        if(job >= njobs) break;
-        const int gi = find_group(groups, ngroups, job);
+        __syncwarp();
+        unsigned long long taken = 0;
+        if(lane == 0) taken = atomicAdd(block_counter, 1ull);
+        taken = __shfl_sync(0xffffffffu, taken, 0);
+        if(taken >= (unsigned long long)end_block) break;
+        const int gi = find_block_group(groups, ngroups, (int)taken);
         const GroupDev &G = groups[gi];
         const EnvDev &e = (staged && gi == gs) ? s_env : *G.env;
-        int local = (int)(job - G.job_base);
+        const int local = ((int)taken - G.blk_base) * G.lanes + lane;
+        if(lane >= G.lanes || local >= G.njobs) continue;
+        const long long job = G.job_base + local;
         int nalpha_eff = e.isingle > 0 ? 1 : e.nalpha;
         int ialpha = e.isingle > 0 ? e.isingle - 1 : local % nalpha_eff;
         int isz = local / nalpha_eff;
@@ -501,11 +506,11 @@ cudaError_t launch_set_counter(unsigned long long *p, unsigned long long v, cuda
 }
 
 namespace {
-template<typename R, int K> cudaError_t launch_trace_k(const GroupDev *groups, int ngroups, long long njobs, void *segs,
+template<typename R, int K> cudaError_t launch_trace_k(const GroupDev *groups, int ngroups, int end_block, void *segs,
                                                        unsigned long long cap, RunCounters *ctr,
-                                                       unsigned long long *job_counter, unsigned int *blk_state,
+                                                       unsigned long long *block_counter, unsigned int *blk_state,
                                                        int grid, int block, cudaStream_t st,
-                                                       unsigned int stage_bytes, int lanes)
+                                                       unsigned int stage_bytes)
 {
     // the ray state is FP64 in both precisions (the mixed precision writes FP32
     // segment records for its FP32 influence kernel): the trajectory, and with it
@@ -518,25 +523,25 @@ template<typename R, int K> cudaError_t launch_trace_k(const GroupDev *groups, i
         attr_set = true;
     }
     if(stage_bytes > STAGE_MAX_BYTES) stage_bytes = STAGE_MAX_BYTES;
-    trace_kernel<double, R, K><<<grid, block, stage_bytes, st>>>(groups, ngroups, njobs, (SegRec<R> *)segs, cap, ctr,
-                                                                 job_counter, blk_state, stage_bytes, lanes);
+    trace_kernel<double, R, K><<<grid, block, stage_bytes, st>>>(groups, ngroups, end_block, (SegRec<R> *)segs, cap,
+                                                                 ctr, block_counter, blk_state, stage_bytes);
     return cudaGetLastError();
 }
 } // namespace
 
-// kind: the profile type of every launched group when all have packed segments
+// rays of blocks [*block_counter, end_block); kind: the profile type of every launched group when all have packed segments
 // (SSP_CLINEAR, SSP_CUBIC, SSP_PCHIP), else 0
-template<typename R> cudaError_t launch_trace(const GroupDev *groups, int ngroups, long long njobs,
+template<typename R> cudaError_t launch_trace(const GroupDev *groups, int ngroups, int end_block,
                                               void *segs, unsigned long long cap, RunCounters *ctr,
-                                              unsigned long long *job_counter, unsigned int *blk_state,
+                                              unsigned long long *block_counter, unsigned int *blk_state,
                                               int grid, int block, cudaStream_t st, unsigned int stage_bytes,
-                                              int lanes, int kind)
+                                              int kind)
 {
     auto f = launch_trace_k<R, 0>;
     if(kind == SSP_CLINEAR) f = launch_trace_k<R, SSP_CLINEAR>;
     else if(kind == SSP_CUBIC) f = launch_trace_k<R, SSP_CUBIC>;
     else if(kind == SSP_PCHIP) f = launch_trace_k<R, SSP_PCHIP>;
-    return f(groups, ngroups, njobs, segs, cap, ctr, job_counter, blk_state, grid, block, st, stage_bytes, lanes);
+    return f(groups, ngroups, end_block, segs, cap, ctr, block_counter, blk_state, grid, block, st, stage_bytes);
 }
 
 cudaError_t launch_influence_mixed(const void *segs, unsigned long long cap, const GroupDev *groups, int ngroups,
@@ -576,12 +581,12 @@ cudaError_t launch_scale(const float2 *acc, float2 *out, const GroupDev *groups,
     return cudaGetLastError();
 }
 
-template cudaError_t launch_trace<float>(const GroupDev *, int, long long, void *, unsigned long long,
+template cudaError_t launch_trace<float>(const GroupDev *, int, int, void *, unsigned long long,
                                          RunCounters *, unsigned long long *, unsigned int *, int, int,
-                                         cudaStream_t, unsigned int, int, int);
-template cudaError_t launch_trace<double>(const GroupDev *, int, long long, void *, unsigned long long,
+                                         cudaStream_t, unsigned int, int);
+template cudaError_t launch_trace<double>(const GroupDev *, int, int, void *, unsigned long long,
                                           RunCounters *, unsigned long long *, unsigned int *, int, int,
-                                          cudaStream_t, unsigned int, int, int);
+                                          cudaStream_t, unsigned int, int);
 template cudaError_t launch_influence<float>(const void *, unsigned long long, const GroupDev *, int,
                                              const double *, float2 *, RunCounters *, bool, bool, int,
                                              cudaStream_t);
