@@ -149,6 +149,26 @@ int64_t field_elems(const Env3Tables &T)
     return (int64_t)T.sz.size() * T.sx.size() * T.sy.size() * T.theta.size() * T.rz.size() * T.rr.size();
 }
 
+// Evenly spaced receiver bearings, so that the influence kernel can go to those
+// near a segment: Env3Dev's theta0, dtheta and theta_full. A spacing is even if
+// every bearing is within 1e-3 of it, which the kernel's margin covers. An open
+// fan wider than half the circle is left out (a segment could reach both ends).
+void even_bearings(const std::vector<double> &deg, Env3Dev &d)
+{
+    const size_t n = deg.size();
+    d.theta0 = d.dtheta = 0.f;
+    d.theta_full = 0;
+    if(n < 2) return;
+    const double step = (deg[n - 1] - deg[0]) / (double)(n - 1);
+    if(!(step > 0.0)) return;
+    for(size_t i = 0; i < n; ++i)
+        if(!(std::fabs(deg[i] - (deg[0] + (double)i * step)) <= 1e-3 * step)) return;
+    d.theta_full = std::fabs(step * (double)n - 360.0) <= 1e-3 * step;
+    if(!d.theta_full && step * (double)(n - 1) > 180.0) return;
+    d.theta0 = (float)((M_PI / 180.0) * std::fmod(deg[0], 360.0));
+    d.dtheta = (float)((M_PI / 180.0) * step);
+}
+
 void prepare3(Run3 *r, cudaStream_t st, uint64_t &h2d)
 {
     if(r->envs.empty()) throw StateError("no 3-D environment: call bhcb_setup3d first");
@@ -219,6 +239,7 @@ void prepare3(Run3 *r, cudaStream_t st, uint64_t &h2d)
         d.nrr = (int)T.rr.size(); d.nrz = (int)T.rz.size(); d.ntheta = (int)T.theta.size();
         d.nalpha = (int)T.alpha.size(); d.nbeta = (int)T.beta.size();
         d.isingle_alpha = T.isingle_alpha; d.isingle_beta = T.isingle_beta;
+        even_bearings(T.theta, d);
         d.dalpha = T.dalpha; d.dbeta = T.dbeta; d.deltas = T.deltas;
         d.box_x = T.box_x; d.box_y = T.box_y; d.box_z = T.box_z; d.freq0 = T.freq0;
         d.gaussian = T.beam_type[0] == 'B' || T.beam_type[0] == 'b';   // IsGaussianGeomInfl

@@ -126,6 +126,11 @@ struct Env3Dev {
     const double *sx, *sy, *rr, *tcs;   // tcs: receiver bearing (cos, sin) pairs
     const double *alpha, *beta;
     const double *acs, *bcs;            // (cos, sin) pairs of alpha and beta, from the host's libm
+    // evenly spaced receiver bearings (rad): the first and the spacing (0: not
+    // even, one bearing, or an open fan wider than half the circle); theta_full:
+    // the fan closes on itself
+    float theta0, dtheta;
+    int32_t theta_full;
     int32_t nx2d;                       // RunType(6) '2': 2-D rays in the bearing planes
     const float *sz, *rz;
     double dalpha, dbeta, deltas, box_x, box_y, box_z, freq0;

@@ -296,14 +296,107 @@ __global__ void __launch_bounds__(64) ray3d_kernel(const GroupDev *__restrict__ 
     }
 }
 
-constexpr int WARPS3 = 4;
+constexpr int WARPS3 = 2;   // the records of 32 segments take 13 KB of shared memory per warp
+
+// What the pair and receiver stages read of a record, in shared memory (the
+// rest of the record only for accepted receivers).
+struct Rec3S {
+    double x0[3], rayt[3], e1[3], e2[3];
+    double rlen, rcp_len;      // segment length, rcp_ulp(rlen)
+    double zlo, zhi, ldiag;
+    double q0[4], dq[4], rcp_q0, rcp_qhat0;
+    float q0f[4], dqf[4], rq0f, rq1f;   // the same in FP32 (mixed precision)
+    // bearings_near: bearing of x0 from the source (in spacings from the first
+    // receiver bearing), its range, the angle kappa between that bearing and the
+    // ray's heading (|sin|, cos), and the bound E + F (distance to x0) on the
+    // horizontal distance from the ray line that a beam reaches; F < 0: none
+    float ib0, r0, sk, ck, E, F;
+};
+
+// Record fields of bearings_near (see there).
+__device__ __forceinline__ void beam_reach(Rec3S &S, const Env3Dev &E, double xs, double ys, double margin)
+{
+    S.F = -1.f;
+    const double th = sqrt(S.rayt[0] * S.rayt[0] + S.rayt[1] * S.rayt[1]);
+    const double ax = S.x0[0] - xs, ay = S.x0[1] - ys, r0 = sqrt(ax * ax + ay * ay);
+    if(!(E.dtheta > 0.f) || !(th > 1.0e-3) || !(r0 > 1.0)) return;
+    const double q00 = fabs(S.q0[0] * S.rcp_q0), q10 = fabs(S.q0[2] * S.rcp_q0);
+    const double q01 = fabs(S.q0[1] * S.rcp_qhat0), q11 = fabs(S.q0[3] * S.rcp_qhat0);
+    const double d00 = fabs(S.dq[0] * S.rcp_q0), d10 = fabs(S.dq[2] * S.rcp_q0);
+    const double d01 = fabs(S.dq[1] * S.rcp_qhat0), d11 = fabs(S.dq[3] * S.rcp_qhat0);
+    const bool gauss = E.gaussian != 0;
+    const double Q = gauss ? max(max(q00, q01), max(q10, q11)) : max(q00 + q01, q10 + q11);
+    const double D = gauss ? max(max(d00, d01), max(d10, d11)) : max(d00 + d01, d10 + d11);
+    const double zm = max(fabs((double)E.rz[0] - S.x0[2]), fabs((double)E.rz[E.nrz - 1] - S.x0[2]));
+    const double w = (gauss ? 4.0 : 1.0) * 1.4142135623730951 * (1.0 + 2.0 * margin) + margin;
+    const double sk = (ay * S.rayt[0] - ax * S.rayt[1]) / (r0 * th), ck = (ax * S.rayt[0] + ay * S.rayt[1]) / (r0 * th);
+    if(!(ck > 0.5)) return;
+    S.ib0 = (atan2f((float)ay, (float)ax) - E.theta0) / E.dtheta;
+    S.r0 = (float)r0;
+    S.sk = (float)fabs(sk);
+    S.ck = (float)ck;
+    S.E = (float)(w * (Q + D * zm * fabs(S.rayt[2]) / S.rlen) + margin);
+    S.F = (float)(w * D / S.rlen);
+}
+
+// The receiver bearings [first, first + count) (modulo ntheta on a closed fan)
+// at range rr that a segment's beam can reach; all of them where nothing
+// smaller follows. For a receiver at angle d from x0's bearing (|d| <= 90
+// degrees, the others are behind the source), its horizontal distance from the
+// ray line is at least rr (sin(|d| + kappa) - sin kappa) - |rr - r0| sin kappa,
+// its distance from x0 at most |rr - r0| + 2 rr sin(|d| / 2), and an accepted
+// one's horizontal distance from the line is at most E + F (distance from x0):
+// n1 and n2 are bounded as in depth_window, q by |q0| + |s| |dq|, and |s| by
+// the distance over the segment length. So accepted receivers have
+// f(d) = sin(d + kappa) - sin kappa - 2 F sin(d / 2) <= G. With kappa <= 60
+// degrees and F <= 0.5 f is concave on [0, 90], so if f(90) > G, f stays above
+// G once it is.
+// Of the 51,984-ray workload's 36 bearings about 4 remain; the pair tests of the
+// other 32 were 45 of the kernel's 55 ms.
+__device__ __forceinline__ void bearings_near(const Rec3S &S, const Env3Dev &E, float rr, int &first, int &count)
+{
+    first = 0;
+    count = E.ntheta;
+    if(!(S.F >= 0.f && S.F <= 0.5f) || !(rr > 1.f)) return;
+    const float G = (S.E + (S.F + S.sk) * fabsf(rr - S.r0)) / rr * 1.002f + 1.0e-5f;
+    const float half = 0.70710678f;   // sin 45 degrees
+    if(!(S.ck - S.sk - 2.f * S.F * half > G)) return;
+    float d = max(E.dtheta, 1.1f * G);
+    for(int it = 0; it < 40; ++it) {
+        if(d >= 1.5707f) return;
+        float sd, cd;
+        __sincosf(d, &sd, &cd);
+        if(sd * S.ck + cd * S.sk - S.sk - 2.f * S.F * __sinf(0.5f * d) > G) break;
+        if(it == 39) return;
+        d *= 1.3f;
+    }
+    const float k = d / E.dtheta + 0.01f;
+    float b = S.ib0;
+    if(!E.theta_full) {   // the turn of the circle nearest to the fan's middle
+        const float turn = 6.28318531f / E.dtheta, mid = 0.5f * (float)(E.ntheta - 1);
+        b -= turn * rintf((b - mid) / turn);
+    }
+    int lo = (int)ceilf(b - k), hi = (int)floorf(b + k);
+    if(E.theta_full) {
+        if(hi - lo + 1 >= E.ntheta) return;
+        first = lo % E.ntheta;
+        if(first < 0) first += E.ntheta;
+        count = max(hi - lo + 1, 0);
+    } else {
+        lo = max(lo, 0);
+        hi = min(hi, E.ntheta - 1);
+        first = lo;
+        count = max(hi - lo + 1, 0);
+    }
+}
 
 // InfluenceGeoCore, 3-D Cartesian (src/influence.hpp:897-1024): beam-window
 // test, then amplitude cnst, weight w, phase and complex delay of one receiver
 struct Contrib3 {
     double cnst, w, ph, dr, di;
 };
-__device__ __forceinline__ bool geo_core3(const SegRec3 &R, double s, double n1, double n2, bool gauss, Contrib3 &o)
+__device__ __forceinline__ bool geo_core3(const Rec3S &R, const SegRec3 &G, double s, double n1, double n2, bool gauss,
+                                          Contrib3 &o)
 {
     double q00 = R.q0[0] + s * R.dq[0], q01 = R.q0[1] + s * R.dq[1];
     double q10 = R.q0[2] + s * R.dq[2], q11 = R.q0[3] + s * R.dq[3];
@@ -321,12 +414,12 @@ __device__ __forceinline__ bool geo_core3(const SegRec3 &R, double s, double n1,
     const double bw = gauss ? 4.0 : 1.0;
     const double dist = gauss ? n1p + n2p : max(n1p, n2p);
     if(dist > bw * 1.0) return false;
-    o.dr = R.tau0r + s * R.dtaur;
-    o.di = R.tau0i + s * R.dtaui;
-    o.cnst = R.cnst_num / sqrt(fabs(qF));
+    o.dr = G.tau0r + s * G.dtaur;
+    o.di = G.tau0i + s * G.dtaui;
+    o.cnst = G.cnst_num / sqrt(fabs(qF));
     o.w = gauss ? exp(FLTD(-0.5) * (n1p * n1p + n2p * n2p)) : (FLTD(1.0) - n1p) * (FLTD(1.0) - n2p);
-    o.ph = R.phase0;
-    if((qF <= 0.0 && R.qold > 0.0) || (qF >= 0.0 && R.qold < 0.0)) o.ph += BHCB_PI / FLTD(2.0);
+    o.ph = G.phase0;
+    if((qF <= 0.0 && G.qold > 0.0) || (qF >= 0.0 && G.qold < 0.0)) o.ph += BHCB_PI / FLTD(2.0);
     return true;
 }
 
@@ -351,15 +444,14 @@ __device__ __forceinline__ float2 tl_field3(const Contrib3 &o, bool gauss, bool 
 // window, amplitude and weight with the SFU's approximations; the delay's
 // phase omega tau is formed and reduced mod 2 pi in FP64, the rest in FP32).
 // Same tests and formulas as geo_core3 + tl_field3.
-__device__ __forceinline__ bool geo_tl3_mixed(const SegRec3 &R, double s, double n1, double n2, bool gauss,
-                                              bool coherent, double omega, float2 &out)
+__device__ __forceinline__ bool geo_tl3_mixed(const Rec3S &R, const SegRec3 &G, double s, double n1, double n2,
+                                              bool gauss, bool coherent, double omega, float2 &out)
 {
     const float sf = (float)s;
-    const float rq0 = (float)R.rcp_q0, rq1 = (float)R.rcp_qhat0;
-    const float q00 = fmaf(sf, (float)R.dq[0], (float)R.q0[0]) * rq0;
-    const float q10 = fmaf(sf, (float)R.dq[2], (float)R.q0[2]) * rq0;
-    const float q01 = fmaf(sf, (float)R.dq[1], (float)R.q0[1]) * rq1;
-    const float q11 = fmaf(sf, (float)R.dq[3], (float)R.q0[3]) * rq1;
+    const float q00 = fmaf(sf, R.dqf[0], R.q0f[0]) * R.rq0f;
+    const float q10 = fmaf(sf, R.dqf[2], R.q0f[2]) * R.rq0f;
+    const float q01 = fmaf(sf, R.dqf[1], R.q0f[1]) * R.rq1f;
+    const float q11 = fmaf(sf, R.dqf[3], R.q0f[3]) * R.rq1f;
     const float qF = q00 * q11 - q10 * q01;
     const float eps2 = (float)(DBL_EPS * DBL_EPS);
     if(q00 * q00 + q10 * q10 < eps2 || q01 * q01 + q11 * q11 < eps2) return false;
@@ -370,13 +462,13 @@ __device__ __forceinline__ bool geo_tl3_mixed(const SegRec3 &R, double s, double
     const float n2p = fabsf((q00 * n2f - q10 * n1f) * iq);
     const float dist = gauss ? n1p + n2p : fmaxf(n1p, n2p);
     if(dist > (gauss ? 4.0f : 1.0f)) return false;
-    const float cnst = (float)R.cnst_num * rsqrtf(fabsf(qF));
+    const float cnst = (float)G.cnst_num * rsqrtf(fabsf(qF));
     const float w = gauss ? __expf(-0.5f * (n1p * n1p + n2p * n2p)) : (1.0f - n1p) * (1.0f - n2p);
-    const float att = __expf((float)(omega * (R.tau0i + s * R.dtaui)));
+    const float att = __expf((float)(omega * (G.tau0i + s * G.dtaui)));
     if(coherent) {
-        float ph = (float)R.phase0;
-        if((qF <= 0.0f && R.qold > 0.0) || (qF >= 0.0f && R.qold < 0.0)) ph += (float)(BHCB_PI / 2.0);
-        const double a = omega * (R.tau0r + s * R.dtaur);
+        float ph = (float)G.phase0;
+        if((qF <= 0.0f && G.qold > 0.0) || (qF >= 0.0f && G.qold < 0.0)) ph += (float)(BHCB_PI / 2.0);
+        const double a = omega * (G.tau0r + s * G.dtaur);
         const float ar = (float)(a - 6.28318530717958647692 * rint(a * 0.15915494309189533577));
         float sa, ca;
         __sincosf(ph - ar, &sa, &ca);
@@ -391,57 +483,90 @@ __device__ __forceinline__ bool geo_tl3_mixed(const SegRec3 &R, double s, double
     return true;
 }
 
-// first index with (double)rz >= z (n if none)
+// first index with (double)rz >= z (n if none); z rounded up to float selects the same
 __device__ __forceinline__ int first_depth_at_or_above(const float *rz, int n, double z)
 {
+    const float zf = __double2float_ru(z);
     int lo = 0, hi = n;
     while(lo < hi) {
         const int m = (lo + hi) >> 1;
-        if((double)rz[m] < z) lo = m + 1; else hi = m;
+        if(__ldg(rz + m) < zf) lo = m + 1; else hi = m;
     }
     return lo;
 }
 // last index with (double)rz <= z (-1 if none)
 __device__ __forceinline__ int last_depth_at_or_below(const float *rz, int n, double z)
 {
+    const float zf = __double2float_rd(z);
     int lo = 0, hi = n;
     while(lo < hi) {
         const int m = (lo + hi) >> 1;
-        if((double)rz[m] <= z) lo = m + 1; else hi = m;
+        if(__ldg(rz + m) <= zf) lo = m + 1; else hi = m;
     }
     return lo - 1;
 }
 
-// A (range, bearing) pair none of whose depths can pass InfluenceGeoCore's
-// beam-window test. With A the row-scaled interpolated q (2x2), the accepted
-// normal offsets satisfy (n1, n2) = A (+-n1', +-n2'), so their length is at
-// most |A|_F |(n1', n2')| <= |A|_F w (w = 4 for Gaussian n1' + n2' <= 4,
-// sqrt 2 for hat max(n1', n2') <= 1). That length is at least the distance
-// between the receivers' vertical line and the ray line, m' / |t_xy|, and
-// |A(s)|_F is convex in s, so its largest value over the depth window is at
-// one of the window's two ends. The margin keeps rounding from dropping a
-// contribution the per-receiver test would accept.
-__device__ __forceinline__ bool pair_outside_beam(const SegRec3 &R, double dxr, double dyr, double mprime,
-                                                  double z_lo, double z_hi, bool gauss)
+// The depths of a (range, bearing) pair's vertical line that InfluenceGeoCore's
+// beam-window test can accept, as [zl, zh] shrunk from the window passed in
+// (false: none). With A = [[q00, q01], [q10, q11]] the row-scaled q at s, the
+// test's normalised offsets (a, b) give the normal offsets n1 = q00 a + q01 b
+// and n2 = q10 a + q11 b. Gaussian beams accept |a| + |b| <= 4, so |n1| <= 4
+// max(|q00|, |q01|); hat beams |a|, |b| <= 1, so |n1| <= |q00| + |q01|; n2
+// likewise. Both bounds are convex in s, which is linear in depth, so over a
+// window they are largest at its ends; n1 and n2 before the absolute value are
+// linear in depth. Two passes: the second has the smaller window's bounds. The
+// margin keeps rounding from dropping a receiver that the test accepts (FP32
+// in the mixed precision).
+// Why: the vertical extent of a beam is set by the spacing of the elevations,
+// 15 times finer than that of the bearings in the 51,984-ray workload, while
+// the window of L_diag is the wider of the two: nearly all 101 depths of every
+// pair, 95 % of them rejected one by one.
+__device__ __forceinline__ bool depth_window(const Rec3S &R, double h, double a1, double a2, bool gauss, double margin,
+                                             double &zl, double &zh)
 {
-    const double th = sqrt(R.rayt[0] * R.rayt[0] + R.rayt[1] * R.rayt[1]);
-    if(!(th > 0.0)) return false;
-    const double h = dxr * R.rayt[0] + dyr * R.rayt[1];
-    double f = 0.0;
+    const double w = (gauss ? 4.0 : 1.0) * (1.0 + margin);
+    const double c1 = R.e1[2], c2 = R.e2[2];
 #pragma unroll
-    for(int e = 0; e < 2; ++e) {
-        const double s = (h + ((e ? z_hi : z_lo) - R.x0[2]) * R.rayt[2]) / R.rlen;
-        const double a0 = (R.q0[0] + s * R.dq[0]) * R.rcp_q0, a2 = (R.q0[2] + s * R.dq[2]) * R.rcp_q0;
-        const double a1 = (R.q0[1] + s * R.dq[1]) * R.rcp_qhat0, a3 = (R.q0[3] + s * R.dq[3]) * R.rcp_qhat0;
-        f = max(f, a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3);
+    for(int pass = 0; pass < 2; ++pass) {
+        double b1 = 0.0, b2 = 0.0, f1[2], f2[2];
+#pragma unroll
+        for(int e = 0; e < 2; ++e) {
+            const double dz = (e ? zh : zl) - R.x0[2];
+            const double s = (h + dz * R.rayt[2]) * R.rcp_len;
+            const double q00 = fabs((R.q0[0] + s * R.dq[0]) * R.rcp_q0), q10 = fabs((R.q0[2] + s * R.dq[2]) * R.rcp_q0);
+            const double q01 = fabs((R.q0[1] + s * R.dq[1]) * R.rcp_qhat0);
+            const double q11 = fabs((R.q0[3] + s * R.dq[3]) * R.rcp_qhat0);
+            b1 = max(b1, gauss ? max(q00, q01) : q00 + q01);
+            b2 = max(b2, gauss ? max(q10, q11) : q10 + q11);
+            f1[e] = a1 + dz * c1;
+            f2[e] = a2 + dz * c2;
+        }
+        b1 = w * b1 + margin;
+        b2 = w * b2 + margin;
+        if((f2[0] > b2 && f2[1] > b2) || (f2[0] < -b2 && f2[1] < -b2)) return false;
+        if((f1[0] > b1 && f1[1] > b1) || (f1[0] < -b1 && f1[1] < -b1)) return false;
+        if(fabs(c1) > 1.0e-3) {
+            const double r = 1.0 / c1, mid = R.x0[2] - a1 * r, half = b1 * fabs(r);
+            zl = max(zl, mid - half);
+            zh = min(zh, mid + half);
+        }
+        if(fabs(c2) > 1.0e-3) {
+            const double r = 1.0 / c2, mid = R.x0[2] - a2 * r, half = b2 * fabs(r);
+            zl = max(zl, mid - half);
+            zh = min(zh, mid + half);
+        }
+        if(!(zl <= zh)) return false;
     }
-    const double w = gauss ? 4.0 : 1.4142135623730951;
-    return mprime > th * w * sqrt(f) * (1.0 + 1e-6) + 1e-9;
+    return true;
 }
 
-// Work is flattened twice per warp: (segment, range, bearing) pairs over the
-// warp's 32 records, then (pair, depth) items over the pairs that survive the
-// bearing rejections, so that every lane evaluates receivers.
+// Work is flattened three times per warp: (segment, range) units over the
+// warp's 32 records, (unit, bearing) pairs over the bearings a beam can reach,
+// then (pair, depth) items over the pairs' depth windows, so that every lane
+// evaluates receivers. Bound by instruction issue. The 51,984-ray workload (287 M
+// contributions, mixed) took 115 ms with every bearing tested and every depth
+// within L_diag evaluated (one item in 18 applied), 55 with depth_window and
+// the records in shared memory, 22.6 with bearings_near.
 // MODE: INFL_TL adds the field; INFL_ARR_COUNT counts the arrival candidates;
 // INFL_ARR_FILL writes them (AddArr's inputs, src/influence.hpp:444-447) with
 // the key (receiver cell, ray, step) that restores the reference's order.
@@ -457,16 +582,21 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
     unsigned long long *cursor, ArrKeyBits kb)
 {
     // per record of the warp's chunk
+    __shared__ Rec3S s_rec[WARPS3][32];
     __shared__ int s_incl[WARPS3][32];
-    __shared__ int s_grp[WARPS3][32];
+    __shared__ int s_grp[WARPS3][32], s_irlo[WARPS3][32];
+    __shared__ const Env3Dev *s_env[WARPS3][32];
     __shared__ long long s_fbase[WARPS3][32];    // field offset of (isz, isx, isy)
     __shared__ double s_xs[WARPS3][32], s_ys[WARPS3][32];
+    // per (record, range) unit of a 32-unit batch: candidate bearings
+    __shared__ int s_uincl[WARPS3][32], s_urec[WARPS3][32], s_uir[WARPS3][32], s_uth[WARPS3][32];
     // per surviving pair of a 32-pair batch
     __shared__ int s_pincl[WARPS3][32];
     __shared__ int s_prec[WARPS3][32], s_piz0[WARPS3][32], s_pmeta[WARPS3][32];
-    __shared__ double s_pdx[WARPS3][32], s_pdy[WARPS3][32];
+    __shared__ double s_ph[WARPS3][32], s_pa1[WARPS3][32], s_pa2[WARPS3][32];
     __shared__ long long s_poff[WARPS3][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double margin = MODE == INFL_TL_MIXED ? 1.0e-3 : 1.0e-6;
     const unsigned long long nchunk = (nseg + 31) / 32;
     unsigned long long nevals = 0;
     for(unsigned long long ch = (unsigned long long)blockIdx.x * WARPS3 + w; ch < nchunk;
@@ -474,18 +604,46 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
         const unsigned long long idx = ch * 32 + lane;
         int n = 0, g = 0;
         if(idx < nseg) {
-            const int job = __ldg(&segs[idx].job);
+            const SegRec3 &R = segs[idx];
+            const int job = __ldg(&R.job);
             if(job >= 0) {
                 g = find_group(groups, ngroups, job);
                 const GroupDev &G = groups[g];
                 const Env3Dev &E = *G.env3;
-                const int lo = __ldg(&segs[idx].ir_lo), hi = __ldg(&segs[idx].ir_hi);
-                n = (hi - lo + 1) * E.ntheta;
+                const int lo = __ldg(&R.ir_lo), hi = __ldg(&R.ir_hi);
+                n = hi - lo + 1;
                 const Job3 J = job_indices3(E, (int)(job - G.job_base));
                 s_fbase[w][lane] = G.field_base
                     + (long long)(((size_t)J.isz * E.nsx + J.isx) * E.nsy + J.isy) * E.ntheta * E.nrz * E.nrr;
                 s_xs[w][lane] = E.sx[J.isx];
                 s_ys[w][lane] = E.sy[J.isy];
+                s_irlo[w][lane] = lo;
+                s_env[w][lane] = &E;
+                Rec3S &S = s_rec[w][lane];
+#pragma unroll
+                for(int i = 0; i < 3; ++i) {
+                    S.x0[i] = R.x0[i];
+                    S.rayt[i] = R.rayt[i];
+                    S.e1[i] = R.e1[i];
+                    S.e2[i] = R.e2[i];
+                }
+                S.rlen = R.rlen;
+                S.rcp_len = rcp_ulp(R.rlen);
+                S.zlo = R.zlo;
+                S.zhi = R.zhi;
+                S.ldiag = R.ldiag;
+#pragma unroll
+                for(int i = 0; i < 4; ++i) {
+                    S.q0[i] = R.q0[i];
+                    S.dq[i] = R.dq[i];
+                    S.q0f[i] = (float)R.q0[i];
+                    S.dqf[i] = (float)R.dq[i];
+                }
+                S.rcp_q0 = R.rcp_q0;
+                S.rcp_qhat0 = R.rcp_qhat0;
+                S.rq0f = (float)R.rcp_q0;
+                S.rq1f = (float)R.rcp_qhat0;
+                beam_reach(S, E, s_xs[w][lane], s_ys[w][lane], margin);
             }
         }
         int incl = n;
@@ -498,22 +656,46 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
         s_grp[w][lane] = g;
         __syncwarp();
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        for(int pb = 0; pb < total; pb += 32) {
+        for(int ub = 0; ub < total; ub += 32) {
+        // ---- unit stage: one (record, range) per lane, the bearings its beam can reach
+        int nb = 0;
+        if(ub + lane < total) {
+            const int k = ub + lane;
+            int lo = 0, hi = 31;   // first record j with incl[j] > k
+            while(lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if(s_incl[w][mid] > k) hi = mid; else lo = mid + 1;
+            }
+            const int j = lo, ir = s_irlo[w][j] + k - (j ? s_incl[w][j - 1] : 0);
+            const Env3Dev &E = *s_env[w][j];
+            bearings_near(s_rec[w][j], E, (float)E.rr[ir], s_uth[w][lane], nb);
+            s_urec[w][lane] = j;
+            s_uir[w][lane] = ir;
+        }
+        int uincl = nb;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, uincl, o);
+            if(lane >= o) uincl += v;
+        }
+        s_uincl[w][lane] = uincl;
+        __syncwarp();
+        const int utotal = __shfl_sync(0xffffffffu, uincl, 31);
+        for(int pb = 0; pb < utotal; pb += 32) {
             // ---- pair stage: bearing rejections and the depth window
             const int k = pb + lane;
             int m = 0;
-            if(k < total) {
-                int lo = 0, hi = 31;   // first record j with incl[j] > k
+            if(k < utotal) {
+                int lo = 0, hi = 31;   // first unit u with uincl[u] > k
                 while(lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if(s_incl[w][mid] > k) hi = mid; else lo = mid + 1;
+                    if(s_uincl[w][mid] > k) hi = mid; else lo = mid + 1;
                 }
-                const int j = lo;
-                const int local = k - (j ? s_incl[w][j - 1] : 0);
-                const SegRec3 &R = segs[ch * 32 + j];
-                const Env3Dev &E = *groups[s_grp[w][j]].env3;
-                const int itheta = local % E.ntheta;
-                const int ir = R.ir_lo + local / E.ntheta;
+                const int u = lo, j = s_urec[w][u], ir = s_uir[w][u];
+                const Rec3S &R = s_rec[w][j];
+                const Env3Dev &E = *s_env[w][j];
+                int itheta = s_uth[w][u] + k - (u ? s_uincl[w][u - 1] : 0);
+                if(itheta >= E.ntheta) itheta -= E.ntheta;
                 const double xsx = s_xs[w][j], xsy = s_ys[w][j];
                 const double tc = E.tcs[2 * itheta], ts = E.tcs[2 * itheta + 1];
                 const double rr = E.rr[ir];
@@ -528,19 +710,25 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
                 keep = keep && !(fabs(nrz) < 1e-9);
                 if(keep) {
                     const double Lz = (gauss ? 4.0 : 1.0) * R.ldiag / fabs(nrz);
-                    const double zmin = R.zlo - Lz, zmax = R.zhi + Lz;
-                    // receiver depths are sorted: the window is the index range [iz0, iz1]
-                    const int iz0 = first_depth_at_or_above(E.rz, E.nrz, zmin);
-                    const int iz1 = last_depth_at_or_below(E.rz, E.nrz, zmax);
-                    if(iz0 <= iz1
-                       && !pair_outside_beam(R, dxr, dyr, mprime, (double)E.rz[iz0], (double)E.rz[iz1], gauss)) {
-                        m = iz1 - iz0 + 1;
-                        s_prec[w][lane] = j;
-                        s_piz0[w][lane] = iz0;
-                        s_pdx[w][lane] = dxr;
-                        s_pdy[w][lane] = dyr;
-                        s_poff[w][lane] = s_fbase[w][j] + (long long)itheta * E.nrz * E.nrr + ir;
-                        s_pmeta[w][lane] = (itheta << 20) | ir;
+                    // receiver depths are sorted: the window is an index range
+                    const float *rz = E.rz;
+                    const int nrz_ = E.nrz;
+                    double zl = max(R.zlo - Lz, (double)rz[0]), zh = min(R.zhi + Lz, (double)rz[nrz_ - 1]);
+                    const double h = dxr * rtx + dyr * rty;
+                    const double a1 = dxr * R.e1[0] + dyr * R.e1[1], a2 = dxr * R.e2[0] + dyr * R.e2[1];
+                    if(zl <= zh && depth_window(R, h, a1, a2, gauss, margin, zl, zh)) {
+                        const int iz0 = first_depth_at_or_above(rz, nrz_, zl);
+                        const int iz1 = last_depth_at_or_below(rz, nrz_, zh);
+                        if(iz0 <= iz1) {
+                            m = iz1 - iz0 + 1;
+                            s_prec[w][lane] = j;
+                            s_piz0[w][lane] = iz0;
+                            s_ph[w][lane] = h;
+                            s_pa1[w][lane] = a1;
+                            s_pa2[w][lane] = a2;
+                            s_poff[w][lane] = s_fbase[w][j] + (long long)itheta * nrz_ * E.nrr + ir;
+                            s_pmeta[w][lane] = (itheta << 20) | ir;
+                        }
                     }
                 }
             }
@@ -563,16 +751,16 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
                 const int pi = lo;
                 const int iz = s_piz0[w][pi] + q - (pi ? s_pincl[w][pi - 1] : 0);
                 const int j = s_prec[w][pi];
+                const Rec3S &S = s_rec[w][j];
                 const SegRec3 &R = segs[ch * 32 + j];
-                const Env3Dev &E = *groups[s_grp[w][j]].env3;
-                const double dxr = s_pdx[w][pi], dyr = s_pdy[w][pi];
-                const double dz = (double)E.rz[iz] - R.x0[2];
-                const double sv = (dxr * R.rayt[0] + dyr * R.rayt[1] + dz * R.rayt[2]) / R.rlen;
-                const double n1 = fabs(dxr * R.e1[0] + dyr * R.e1[1] + dz * R.e1[2]);
-                const double n2 = fabs(dxr * R.e2[0] + dyr * R.e2[1] + dz * R.e2[2]);
+                const Env3Dev &E = *s_env[w][j];
+                const double dz = (double)E.rz[iz] - S.x0[2];
+                const double sv = quot_rn(s_ph[w][pi] + dz * S.rayt[2], S.rlen, S.rcp_len);
+                const double n1 = fabs(s_pa1[w][pi] + dz * S.e1[2]);
+                const double n2 = fabs(s_pa2[w][pi] + dz * S.e2[2]);
                 if(MODE == INFL_TL_MIXED) {
                     float2 v;
-                    if(!geo_tl3_mixed(R, sv, n1, n2, E.gaussian != 0, E.coherent != 0,
+                    if(!geo_tl3_mixed(S, R, sv, n1, n2, E.gaussian != 0, E.coherent != 0,
                                       FLTD(2.0) * BHCB_PI * E.freq0, v))
                         continue;
                     ++nevals;
@@ -580,7 +768,7 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
                     continue;
                 }
                 Contrib3 o;
-                if(!geo_core3(R, sv, n1, n2, E.gaussian != 0, o)) continue;
+                if(!geo_core3(S, R, sv, n1, n2, E.gaussian != 0, o)) continue;
                 ++nevals;
                 const long long cell = s_poff[w][pi] + (long long)iz * E.nrr;
                 if(MODE == INFL_TL) {
@@ -631,6 +819,7 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
                 }
             }
             __syncwarp();
+        }
         }
         __syncwarp();
     }
@@ -695,10 +884,12 @@ cudaError_t launch_trace3d(const GroupDev *groups, int ngroups, long long job_en
     return cudaGetLastError();
 }
 
+// grid: CTAs of four warps
 cudaError_t launch_influence3d(const SegRec3 *segs, unsigned long long nseg, const GroupDev *groups, int ngroups,
                                float2 *field, RunCounters *ctr, int grid, cudaStream_t st, bool mixed)
 {
     if(nseg == 0) return cudaSuccess;
+    grid = grid * 4 / WARPS3;
     if(mixed)
         influence3d_kernel<INFL_TL_MIXED><<<grid, 32 * WARPS3, 0, st>>>(segs, nseg, groups, ngroups, field, ctr,
                                                                          nullptr, nullptr, nullptr, 0, nullptr,
@@ -717,6 +908,7 @@ cudaError_t launch_arr_gather3d(const SegRec3 *segs, unsigned long long nseg, co
                                 ArrKeyBits kb, int grid, cudaStream_t st)
 {
     if(nseg == 0) return cudaSuccess;
+    grid = grid * 4 / WARPS3;
     if(kb.eigen) {
         if(count)
             influence3d_kernel<INFL_EIG_COUNT><<<grid, 32 * WARPS3, 0, st>>>(segs, nseg, groups, ngroups, nullptr,
