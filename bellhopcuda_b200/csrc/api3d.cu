@@ -39,8 +39,8 @@ cudaError_t launch_influence_nx(const void *, unsigned long long, const GroupDev
                                 int, cudaStream_t);
 cudaError_t launch_scale_nx(float2 *, const GroupDev *, int, int, cudaStream_t);
 size_t nx_record_bytes();
-cudaError_t launch_trace3d(const GroupDev *, int, long long, SegRec3 *, unsigned long long, RunCounters *,
-                           unsigned long long *, int, cudaStream_t);
+cudaError_t launch_trace3d(const GroupDev *, int, long long, long long, SegRec3 *, unsigned long long, RunCounters *,
+                           unsigned long long *, int, int, cudaStream_t);
 cudaError_t launch_influence3d(const SegRec3 *, unsigned long long, const GroupDev *, int, float2 *, RunCounters *,
                                int, cudaStream_t, bool);
 cudaError_t launch_sqrt3d(float2 *, long long, int, cudaStream_t);
@@ -99,6 +99,7 @@ struct Run3 {
     bool rayrun = false;
     std::vector<RaySet3> raysets;     // per environment
     bool raycen = false;              // geometric beams in ray-centred coordinates ('g', 'b')
+    int kind = 0;                    // 1: every environment hexahedral, 2: none, 0: both
     bool nx2d = false;                // N x 2-D rays (RunType(6) '2')
     bool mixed = false;               // Cartesian TL contributions in mixed precision (BHCB_PREC_MIXED)
     int sm_count = 148;
@@ -263,6 +264,11 @@ void prepare3(Run3 *r, cudaStream_t st, uint64_t &h2d)
         r->njobs += nj;
         r->total_field += S.field_n;
     }
+    r->kind = 0;
+    size_t nhex = 0;
+    for(const Env3Dev &d : envdev) nhex += d.hex ? 1 : 0;
+    if(nhex == envdev.size()) r->kind = 1;
+    else if(nhex == 0) r->kind = 2;
     const size_t env_off = A.put(envdev);
     r->arena.ensure(A.bytes.size());
     void *ab = r->arena.p;
@@ -535,8 +541,8 @@ void run_jobs(Run3 *r, long long j0, long long j1, cudaStream_t st, int sm_count
             CK(launch_trace3d_rc((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), j1, (XSeg3 *)r->segs.p,
                                  r->seg_cap, ctr, jc, tgrid, st));
         else
-            CK(launch_trace3d((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), j1, (SegRec3 *)r->segs.p,
-                              r->seg_cap, ctr, jc, tgrid, st));
+            CK(launch_trace3d((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), nj, j1, (SegRec3 *)r->segs.p,
+                              r->seg_cap, ctr, jc, sm_count, r->kind, st));
         CK(cudaEventRecord(e1, st));
         RunCounters rc{};
         CK(cudaMemcpyAsync(&rc, ctr, sizeof rc, cudaMemcpyDeviceToHost, st));

@@ -21,6 +21,8 @@
 //                     1596-1606); coherent 3-D fields are not scaled.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "bhcb_internal.h"
 #include "device_math.cuh"
 #include "trace2d.cuh"
@@ -63,60 +65,78 @@ struct Infl3 {
     double ratio1, rcp_q0, rcp_qhat0;
     V3 xs;
     int ir;
+    double r;            // horizontal distance of the last point from the source
+    double rr;           // the receiver range E.rr[ir]
 };
 
 __device__ __forceinline__ double row_len(const M2 &q, int row, double s)
 {
     const double a = q.m[0][row] * s, b = q.m[1][row] * s;
-    return sqrt(a * a + b * b);
+    return sqrt_any(a * a + b * b);
 }
 
-// Step_InfluenceGeoCart, 3-D, up to the receiver loop (src/influence.hpp:1201-1292)
+// Step_InfluenceGeoCart, 3-D, up to the receiver loop (src/influence.hpp:1201-1292).
+// What only a segment that brackets a receiver range needs (ray normals, beam
+// width bound) is computed after the range walk. cphi, sphi: of P1.phi.
 __device__ __forceinline__ bool infl_prologue3(const Ray3 &P0, const Ray3 &P1, Infl3 &inf, const Env3Dev &E,
-                                               int job, int is, SegRec3 &rec)
+                                               double cphi, double sphi, int job, int is, SegRec3 &rec)
 {
-    const double ax = P0.x.x - inf.xs.x, ay = P0.x.y - inf.xs.y;
     const double bx = P1.x.x - inf.xs.x, by = P1.x.y - inf.xs.y;
-    const double rA = sqrt(ax * ax + ay * ay), rB = sqrt(bx * bx + by * by);
+    const double rA = inf.r, rB = sqrt_any(bx * bx + by * by);
+    inf.r = rB;
     if(fabs(rA - rB) <= 1.0e3 * spacing_d(rA)) return false;   // IsDuplicatePoint(rB, rA)
-    if(is == 0) inf.ir = rB > rA ? 0 : E.nrr - 1;
+    if(is == 0) {
+        inf.ir = rB > rA ? 0 : E.nrr - 1;
+        inf.rr = E.rr[inf.ir];
+    }
     V3 rayt = sub3(P1.x, P0.x);
-    const double rlen = len3(rayt);
-    if(rlen <= 1.0e3 * spacing_d(P1.x.x)) return false;
-    rayt = v3(rayt.x / rlen, rayt.y / rlen, rayt.z / rlen);
-    V3 e1, e2;
-    ray_normal(rayt, P1.phi, true, 1.0, e1, e2);
+    const double dd = dot3(rayt, rayt);
+    // |d| > 1e-12 |x| is above the threshold of 1000 spacings (2.3e-13 |x| at most)
+    const bool long_seg = dd > 1.0e-24 * (P1.x.x * P1.x.x) && dd > 1.0e-200;
+    const double rlen = long_seg ? sqrt_rn(dd) : sqrt(dd);
+    if(!long_seg && rlen <= 1.0e3 * spacing_d(P1.x.x)) return false;
     const double phaseq = m2_det(P0.q);
     if((phaseq <= 0.0 && inf.qOld > 0.0) || (phaseq >= 0.0 && inf.qOld < 0.0)) inf.phase += BHCB_PI / FLTD(2.0);
     inf.qOld = phaseq;
-    const double l1 = max(row_len(P0.q, 0, inf.rcp_q0), row_len(P1.q, 0, inf.rcp_q0));
-    const double l2 = max(row_len(P0.q, 1, inf.rcp_qhat0), row_len(P1.q, 1, inf.rcp_qhat0));
-    const double ldiag = sqrt(l1 * l1 + l2 * l2);
 
     // receiver-range walk (src/influence.hpp:1294-1297, 1386-1399): the
     // bracketed ranges of one segment are contiguous
     const double *rr = E.rr;
+    const int nrr = E.nrr;
     const double rmin = min(rA, rB), rmax = max(rA, rB);
-    int lo = 0x7fffffff, hi = -1;
+    int lo = 0x7fffffff, hi = -1, ir = inf.ir;
+    double r = inf.rr;
     for(;;) {
-        const double r = rr[inf.ir];
         if(r >= rmin && r < rmax) {
-            lo = min(lo, inf.ir);
-            hi = max(hi, inf.ir);
+            lo = min(lo, ir);
+            hi = max(hi, ir);
         }
         int irTT;
+        double rTT;
         if(rB > r) {
-            if(inf.ir >= E.nrr - 1) break;
-            irTT = inf.ir + 1;
-            if(rr[irTT] >= rB) break;
+            if(ir >= nrr - 1) break;
+            irTT = ir + 1;
+            rTT = rr[irTT];
+            if(rTT >= rB) break;
         } else {
-            if(inf.ir <= 0) break;
-            irTT = inf.ir - 1;
-            if(rr[irTT] <= rB) break;
+            if(ir <= 0) break;
+            irTT = ir - 1;
+            rTT = rr[irTT];
+            if(rTT <= rB) break;
         }
-        inf.ir = irTT;
+        ir = irTT;
+        r = rTT;
     }
+    inf.ir = ir;
+    inf.rr = r;
     if(hi < 0) return false;
+    const double rl = rcp_ulp(rlen);
+    rayt = v3(quot_rn(rayt.x, rlen, rl), quot_rn(rayt.y, rlen, rl), quot_rn(rayt.z, rlen, rl));
+    V3 e1, e2;
+    ray_normal_unit(rayt, P1.phi, cphi, sphi, e1, e2);
+    const double l1 = max(row_len(P0.q, 0, inf.rcp_q0), row_len(P1.q, 0, inf.rcp_q0));
+    const double l2 = max(row_len(P0.q, 1, inf.rcp_qhat0), row_len(P1.q, 1, inf.rcp_qhat0));
+    const double ldiag = sqrt_any(l1 * l1 + l2 * l2);
     rec.x0[0] = P0.x.x; rec.x0[1] = P0.x.y; rec.x0[2] = P0.x.z;
     rec.tau0r = P0.taur;
     rec.tau0i = P0.taui;
@@ -148,20 +168,29 @@ __device__ __forceinline__ bool infl_prologue3(const Ray3 &P0, const Ray3 &P1, I
     return true;
 }
 
-__global__ void __launch_bounds__(64) trace3d_kernel(const GroupDev *__restrict__ groups, int ngroups,
-                                                     long long job_end, SegRec3 *segs, unsigned long long cap,
-                                                     RunCounters *ctr, unsigned long long *job_counter)
+// M: 1 when every group of the launch has the hexahedral grid, 2 when every
+// one has a 1-D profile (Ray3Walk), 0 for a mixture (general step). Warps take
+// `lanes` consecutive jobs at a time.
+template<int M> __global__ void __launch_bounds__(64) trace3d_kernel(const GroupDev *__restrict__ groups, int ngroups,
+                                                                     long long job_end, SegRec3 *segs,
+                                                                     unsigned long long cap, RunCounters *ctr,
+                                                                     unsigned long long *job_counter, int lanes)
 {
+    const int lane = (int)(threadIdx.x & 31);
     for(;;) {
-        const long long job = (long long)atomicAdd(job_counter, 1ull);
-        if(job >= job_end) break;
+        __syncwarp();
+        unsigned long long base = 0;
+        if(lane == 0) base = atomicAdd(job_counter, (unsigned long long)lanes);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if((long long)base >= job_end) break;
+        const long long job = (long long)base + lane;
+        if(lane >= lanes || job >= job_end) continue;
         const GroupDev &G = groups[find_group(groups, ngroups, job)];
         const Env3Dev &E = *G.env3;
         const Job3 J = job_indices3(E, (int)(job - G.job_base));
         if(J.isz >= E.nsz) { run_error(ctr, ERR_RAYINIT); continue; }
         RayState3 st;
         if(!ray_init3d(E, J, st, ctr)) continue;
-        Ray3 &p0 = st.p0;
         Ray3 p1, p2;
         const double alpha = st.alpha, c = st.c;
         // ---- Init_Influence (src/influence.hpp:525-644), 3-D Cartesian geometric
@@ -172,27 +201,39 @@ __global__ void __launch_bounds__(64) trace3d_kernel(const GroupDev *__restrict_
         inf.rcp_q0 = E.dalpha / c;
         inf.rcp_qhat0 = fabs(cos(alpha)) * E.dbeta / c;
         inf.phase = 0.0;
-        inf.qOld = m2_det(p0.q);
-        inf.xs = p0.x;
+        inf.qOld = m2_det(st.p0.q);
+        inf.xs = st.p0.x;
         inf.ir = bsearch_gt(E.rr, E.nrr, 0.0);
+        inf.r = 0.0;
+        inf.rr = E.rr[inf.ir];
 
         int small = 0, is = 0;
         bool overflow = false;
-        unsigned long long nsteps = 0;
+        unsigned int nsteps = 0;
         Cursor3 cur;
+        auto influence = [&](const Ray3 &a, const Ray3 &b, double cp, double sp) {
+            SegRec3 rec;
+            if(infl_prologue3(a, b, inf, E, cp, sp, (int)job, is, rec)) emit_seg3(rec, segs, cap, ctr, cur, overflow);
+            ++is;
+        };
+        Ray3Walk<M == 1> ray;
+        if constexpr(M != 0) ray.init(E, st, ctr);
         for(;;) {
             if((nsteps & 31) == 0 && __ldcg(&ctr->err_bits) != 0u) break;
-            const bool two = ray_update3d(st, p1, p2, small, E, ctr);
             ++nsteps;
-            SegRec3 rec;
-            if(infl_prologue3(p0, p1, inf, E, (int)job, is, rec)) emit_seg3(rec, segs, cap, ctr, cur, overflow);
-            ++is;
-            if(two) {
-                if(infl_prologue3(p1, p2, inf, E, (int)job, is, rec)) emit_seg3(rec, segs, cap, ctr, cur, overflow);
-                p0 = p2;
-                ++is;
+            if constexpr(M != 0) {
+                const int hit = ray.step(p1, ctr);
+                influence(ray.p0, p1, ray.cphi, ray.sphi);
+                ray.p0 = p1;
+                if(hit) {
+                    ray.reflect(hit, ctr);
+                    ++is;   // the reflected point is at the same place: a duplicate for the influence
+                }
             } else {
-                p0 = p1;
+                const bool two = ray_update3d(st, p1, p2, small, E, ctr);
+                influence(st.p0, p1, cos(p1.phi), sin(p1.phi));
+                if(two) influence(p1, p2, cos(p2.phi), sin(p2.phi));
+                st.p0 = two ? p2 : p1;
             }
             if(overflow) {
                 atomicMin(&ctr->overflow_job, (unsigned int)job);
@@ -200,14 +241,18 @@ __global__ void __launch_bounds__(64) trace3d_kernel(const GroupDev *__restrict_
                 break;
             }
             // ---- RayTerminate (src/trace.hpp:391-477), 3-D
-            if(ray_stops3d(st, small, E)) break;
+            if constexpr(M != 0) {
+                if(ray.stops()) break;
+            } else {
+                if(ray_stops3d(st, small, E)) break;
+            }
             if(is >= MAXN_STEPS - 3) {
                 run_warn(ctr, WARN_ONERAY_OUTOFMEMORY);
                 break;
             }
         }
         for(; cur.next < cur.end; ++cur.next) segs[cur.next].job = -1;
-        atomicAdd(&ctr->nsteps, nsteps);
+        atomicAdd(&ctr->nsteps, (unsigned long long)nsteps);
     }
 }
 
@@ -876,11 +921,16 @@ cudaError_t launch_rays3d(const GroupDev *groups, int ngroups, const long long *
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace3d(const GroupDev *groups, int ngroups, long long job_end, SegRec3 *segs,
-                           unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, int grid,
-                           cudaStream_t st)
+// rays per warp for njobs rays (lanes3), the trace of jobs [*job_counter, job_end)
+cudaError_t launch_trace3d(const GroupDev *groups, int ngroups, long long njobs, long long job_end, SegRec3 *segs,
+                           unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, int sm_count,
+                           int kind, cudaStream_t st)
 {
-    trace3d_kernel<<<grid, 64, 0, st>>>(groups, ngroups, job_end, segs, cap, ctr, job_counter);
+    const int lanes = lanes3(njobs, sm_count);
+    const long long warps = (njobs + lanes - 1) / lanes;
+    const int grid = (int)std::max(1LL, std::min<long long>((warps + 1) / 2, (long long)sm_count * 16));
+    auto k = kind == 1 ? trace3d_kernel<1> : kind == 2 ? trace3d_kernel<2> : trace3d_kernel<0>;
+    k<<<grid, 64, 0, st>>>(groups, ngroups, job_end, segs, cap, ctr, job_counter, lanes);
     return cudaGetLastError();
 }
 
