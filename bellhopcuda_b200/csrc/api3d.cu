@@ -30,13 +30,13 @@ cudaError_t launch_trace3d_rc(const GroupDev *, int, long long, XSeg3 *, unsigne
                               unsigned long long *, int, cudaStream_t);
 cudaError_t launch_influence3d_rc(const XSeg3 *, unsigned long long, const GroupDev *, int, float2 *, RunCounters *,
                                   int, int, cudaStream_t);
-cudaError_t launch_trace_nx(const GroupDev *, int, long long, void *, unsigned long long, RunCounters *,
-                            unsigned long long *, int, cudaStream_t);
+cudaError_t launch_trace_nx(const GroupDev *, int, long long, long long, void *, unsigned long long, RunCounters *,
+                            unsigned long long *, int, int, cudaStream_t);
 cudaError_t launch_arr_gather_nx(const void *, unsigned long long, const GroupDev *, int, bool, ArrCand *,
                                  uint64_t *, uint32_t *, unsigned long long, unsigned long long *, RunCounters *,
                                  ArrKeyBits, int, cudaStream_t);
 cudaError_t launch_influence_nx(const void *, unsigned long long, const GroupDev *, int, float2 *, RunCounters *, int,
-                                int, cudaStream_t);
+                                cudaStream_t);
 cudaError_t launch_scale_nx(float2 *, const GroupDev *, int, int, cudaStream_t);
 size_t nx_record_bytes();
 cudaError_t launch_trace3d(const GroupDev *, int, long long, long long, SegRec3 *, unsigned long long, RunCounters *,
@@ -535,8 +535,8 @@ void run_jobs(Run3 *r, long long j0, long long j1, cudaStream_t st, int sm_count
         const long long nj = j1 - j0;
         const int tgrid = (int)std::max<long long>(1, std::min<long long>((nj + 63) / 64, (long long)sm_count * 16));
         if(r->nx2d)
-            CK(launch_trace_nx((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), j1, r->segs.p, r->seg_cap,
-                               ctr, jc, tgrid, st));
+            CK(launch_trace_nx((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), nj, j1, r->segs.p, r->seg_cap,
+                               ctr, jc, sm_count, r->kind, st));
         else if(r->raycen)
             CK(launch_trace3d_rc((const GroupDev *)r->groups_d.p, (int)r->groups_h.size(), j1, (XSeg3 *)r->segs.p,
                                  r->seg_cap, ctr, jc, tgrid, st));
@@ -580,10 +580,8 @@ void run_jobs(Run3 *r, long long j0, long long j1, cudaStream_t st, int sm_count
             return;
         }
         if(rc.err_bits == 0 && r->nx2d) {
-            int nz = 1;
-            for(const auto &S : r->envs) nz = std::max(nz, (int)S.T.rz.size());
             CK(launch_influence_nx(r->segs.p, nseg, (const GroupDev *)r->groups_d.p, (int)r->groups_h.size(),
-                                   (float2 *)r->field.p, ctr, nz, sm_count * 16, st));
+                                   (float2 *)r->field.p, ctr, sm_count * 16, st));
         } else if(rc.err_bits == 0 && r->raycen) {
             int nzt = 1;   // (depth, bearing) pairs per record, the most of the batch
             for(const auto &S : r->envs) nzt = std::max(nzt, (int)(S.T.rz.size() * S.T.theta.size()));

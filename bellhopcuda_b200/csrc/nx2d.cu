@@ -17,7 +17,7 @@
 //                       of the Nx2D path and the sequential part of the 2-D
 //                       influence; one record per segment that brackets
 //                       receiver ranges.
-//  influence_nx_kernel  one thread per (record, receiver depth); contributions
+//  influence_nx_kernel  32 records per warp, their receivers flattened; contributions
 //                       added into the [isz][isx][isy][itheta][iz][ir] field.
 //  scale_nx_kernel      ScalePressure, 2-D form (src/influence.hpp:1556-1627).
 //
@@ -31,12 +31,15 @@
 // bits follow the reference's own arithmetic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "bhcb_internal.h"
 #include "device_math.cuh"
 #include "trace2d.cuh"
 #include "influence2d.cuh"
 #include "ray2d.cuh"
 #include "trace3d.cuh"
+#include "walk3d.cuh"
 
 namespace bhcb {
 
@@ -297,6 +300,30 @@ __device__ bool ray_init_nx(const Env3Dev &E, const Job3 &J, RayStateN &st, RunC
     return true;
 }
 
+// The reflection of p1 into p2 off boundary b (RayUpdate, src/trace.hpp:318-341)
+__device__ void reflect_at_nx(const RayN &p1, RayN &p2, const Bd3 &b, bool tr, const Env3Dev &E, const OrgN &org,
+                              Seg3 &iSeg, RunCounters *ctr)
+{
+    const V3 x_o = to_ocean_x(p1.x, org);
+    V3 nI = b.n;
+    double kappa = 0.0;
+    if(tr ? E.top_curv : E.bot_curv) {   // curvilinear grid (src/trace.hpp:318-341)
+        const Bdry3PtDev *bd = tr ? E.btop : E.bbot;
+        const int ny = tr ? E.top_ny : E.bot_ny;
+        const double s1 = (x_o.x - b.x.x) / (b.xmax - b.xmin), s2 = (x_o.y - b.x.y) / (b.ymax - b.ymin);
+        const double m1 = 1.0 - s1, m2 = 1.0 - s2;
+        const Bdry3PtDev &d00 = bd[(size_t)b.ix * ny + b.iy], &d01 = bd[(size_t)b.ix * ny + b.iy + 1];
+        const Bdry3PtDev &d10 = bd[(size_t)(b.ix + 1) * ny + b.iy], &d11 = bd[(size_t)(b.ix + 1) * ny + b.iy + 1];
+        nI = v3(d00.noden[0] * m1 * m2 + d10.noden[0] * s1 * m2 + d11.noden[0] * s1 * s2 + d01.noden[0] * m1 * s2,
+                d00.noden[1] * m1 * m2 + d10.noden[1] * s1 * m2 + d11.noden[1] * s1 * s2 + d01.noden[1] * m1 * s2,
+                d00.noden[2] * m1 * m2 + d10.noden[2] * s1 * m2 + d11.noden[2] * s1 * s2 + d01.noden[2] * m1 * s2);
+        const double tx = org.tx, ty = org.ty;
+        kappa = d00.kxx * tx * tx + FLTD(2.0) * d00.kxy * tx * ty + d00.kyy * ty * ty;
+        if(tr) kappa = -kappa;
+    }
+    reflect_nx(p1, p2, tr ? E.top : E.bot, tr, nI, kappa, E, org, iSeg, ctr);
+}
+
 // RayUpdate, Nx2D (src/trace.hpp:274-381)
 __device__ bool ray_update_nx(RayStateN &st, RayN &p1, RayN &p2, int &small, const Env3Dev &E, RunCounters *ctr)
 {
@@ -307,24 +334,7 @@ __device__ bool ray_update_nx(RayStateN &st, RayN &p1, RayN &p2, int &small, con
     get_bdry_seg3(x_o, t_o, st.bot, E.bbot, E.bot_nx, E.bot_ny, false, false, ctr);
     const bool two = tr || br;
     if(two) {
-        const Bd3 &b = tr ? st.top : st.bot;
-        V3 nI = b.n;
-        double kappa = 0.0;
-        if(tr ? E.top_curv : E.bot_curv) {   // curvilinear grid (src/trace.hpp:318-341)
-            const Bdry3PtDev *bd = tr ? E.btop : E.bbot;
-            const int ny = tr ? E.top_ny : E.bot_ny;
-            const double s1 = (x_o.x - b.x.x) / (b.xmax - b.xmin), s2 = (x_o.y - b.x.y) / (b.ymax - b.ymin);
-            const double m1 = 1.0 - s1, m2 = 1.0 - s2;
-            const Bdry3PtDev &d00 = bd[(size_t)b.ix * ny + b.iy], &d01 = bd[(size_t)b.ix * ny + b.iy + 1];
-            const Bdry3PtDev &d10 = bd[(size_t)(b.ix + 1) * ny + b.iy], &d11 = bd[(size_t)(b.ix + 1) * ny + b.iy + 1];
-            nI = v3(d00.noden[0] * m1 * m2 + d10.noden[0] * s1 * m2 + d11.noden[0] * s1 * s2 + d01.noden[0] * m1 * s2,
-                    d00.noden[1] * m1 * m2 + d10.noden[1] * s1 * m2 + d11.noden[1] * s1 * s2 + d01.noden[1] * m1 * s2,
-                    d00.noden[2] * m1 * m2 + d10.noden[2] * s1 * m2 + d11.noden[2] * s1 * s2 + d01.noden[2] * m1 * s2);
-            const double tx = st.org.tx, ty = st.org.ty;
-            kappa = d00.kxx * tx * tx + FLTD(2.0) * d00.kxy * tx * ty + d00.kyy * ty * ty;
-            if(tr) kappa = -kappa;
-        }
-        reflect_nx(p1, p2, tr ? E.top : E.bot, tr, nI, kappa, E, st.org, st.iSeg, ctr);
+        reflect_at_nx(p1, p2, tr ? st.top : st.bot, tr, E, st.org, st.iSeg, ctr);
     }
     return two;
 }
@@ -340,6 +350,164 @@ __device__ __forceinline__ bool ray_stops_nx(const RayStateN &st, int small, con
     const bool lost = st.p0.Amp < FLTD(0.005);
     return leftbox || lost || esc0 || escN || small > 50;
 }
+
+// called with copies of the state: long and seldom taken
+static __device__ __noinline__ void reflect_cold_nx(const RayN &p1, RayN &p2, const Bd3 &b, bool tr, const Env3Dev *E,
+                                                    const OrgN &org, Seg3 &iSeg, RunCounters *ctr)
+{
+    reflect_at_nx(p1, p2, b, tr, *E, org, iSeg, ctr);
+}
+
+// The Nx2D ray over Walk3: ray_update_nx and ray_stops_nx with what the ray
+// carries at hand (walk3d.cuh has the reasons). 12,996 rays through the
+// hexahedral ocean: trace 22 -> 16.5 ms, 793 rays 19.5 -> 7, the same step counts.
+template<bool HEX> struct RayNWalk {
+    Walk3<HEX> w;
+    RayN p0;
+    OrgN org;
+    Prof3 o0;                        // the profile at p0
+    double minx, miny, maxx, maxy;
+    double rt;                       // reciprocal of the larger radial component
+    int small;
+    bool low, inside;
+
+    __device__ __forceinline__ void init(const Env3Dev &E, const RayStateN &st, RunCounters *ctr)
+    {
+        w.init(E, st.org.xs, st.top, st.bot, st.iSeg, ctr);
+        p0 = st.p0;
+        org = st.org;
+        minx = st.minx; miny = st.miny; maxx = st.maxx; maxy = st.maxy;
+        rt = rcp_ulp(fabs(org.tx) >= fabs(org.ty) ? org.tx : org.ty);
+        small = 0;
+        low = p0.Amp < FLTD(0.005);
+        inside = false;
+        w.eval(to_ocean_x(p0.x, org), to_ocean_t(p0.t, org), o0, ctr);
+    }
+    // the gradient projected on the plane (eval_ssp_nx)
+    __device__ __forceinline__ V2<double> grad(const Prof3 &o) const
+    {
+        return mk2(org.tx * o.g.x + org.ty * o.g.y, o.g.z);
+    }
+    __device__ __forceinline__ V2<double> to_ray(V3 x, V2<double> t, int snap, RunCounters *ctr) const
+    {
+        if(snap < -2 || snap == -1 || snap >= 2) {
+            V2<double> r;
+            r.y = x.z;
+            r.x = fabs(org.tx) >= fabs(org.ty) ? quot_rn(x.x - org.xs.x, org.tx, rt) : quot_rn(x.y - org.xs.y, org.ty, rt);
+            return r;
+        }
+        return to_ray_x(x, org, t, snap, ctr);
+    }
+    // step_nx and the boundary segments; returns the boundary to reflect at
+    __device__ __forceinline__ int step(RayN &r2, RunCounters *ctr)
+    {
+        const V2<double> t0 = p0.t, x0 = p0.x;
+        const Seg3 s0 = w.s;
+        const Prof3 a = o0;
+        const double c0 = a.c, csq0 = c0 * c0;
+        const V2<double> ga = grad(a);
+        const double cnn0 = a.czz * t0.x * t0.x;
+        const V2<double> pq0p = scl2(-cnn0, p0.q), pq0q = scl2(c0, p0.p);
+        const V2<double> u0 = scl2(c0, t0);
+        const V3 x_o = to_ocean_x(x0, org);
+        bool tr = false, br = false;
+        w.begin();
+        double h = w.deltas, halfh = 0.0, w0 = 0.0, w1 = 0.0, cnn1 = 0.0;
+        V2<double> u = u0, pm = p0.p, qm = p0.q, gb = ga;
+        Prof3 b = a;
+        // one copy of the crossing tests and of the evaluation (Ray3Walk::step)
+#pragma unroll 1
+        for(int pass = 0;; ++pass) {
+            int snap;
+            V3 x2_o;
+            w.cross(pass == 2, x_o, to_ocean_t(u, org), h, x2_o, tr, br, s0, snap, small, ctr);
+            if(pass == 1) {
+                w1 = div_rn(h, 2.0 * halfh);
+                w0 = 1.0 - w1;
+                u = add2(scl2(w0, u0), scl2(w1, u));
+                continue;
+            }
+            double k;
+            V2<double> x;
+            if(pass == 0) {
+                halfh = k = 0.5 * h;
+                x = add2(x0, scl2(halfh, u0));
+            } else {
+                k = h * w0;
+                x = to_ray(x2_o, u, snap, ctr);
+            }
+            V2<double> t = mk2(HEX ? t0.x - quot_rn(k * ga.x, csq0, a.rcsq) : t0.x, t0.y - quot_rn(k * ga.y, csq0, a.rcsq));
+            if(pass == 2) {
+                const double hw1 = h * w1, csq1 = b.c * b.c;
+                if(HEX) t.x = t.x - quot_rn(hw1 * gb.x, csq1, b.rcsq);
+                t.y = t.y - quot_rn(hw1 * gb.y, csq1, b.rcsq);
+                const Cx<double> d0 = a.ci == 0.0 ? cx<double>(quot_rn(k, c0, a.rc), 0.0)
+                                                  : rdivc(k, cx<double>(c0, a.ci));
+                const Cx<double> d1 = b.ci == 0.0 ? cx<double>(quot_rn(hw1, b.c, b.rc), 0.0)
+                                                  : rdivc(hw1, cx<double>(b.c, b.ci));
+                r2.taur = p0.taur + d0.r + d1.r;
+                r2.taui = p0.taui + d0.i + d1.i;
+                const V2<double> pq1p = scl2(-cnn1, qm), pq1q = scl2(b.c, pm);
+                r2.p = HEX ? p0.p : add2(add2(p0.p, scl2(k, pq0p)), scl2(hw1, pq1p));
+                r2.q = add2(add2(p0.q, scl2(k, pq0q)), scl2(hw1, pq1q));
+                r2.x = x;
+                r2.t = t;
+            }
+            Prof3 o;
+            w.eval(to_ocean_x(x, org), to_ocean_t(t, org), o, ctr);
+            if(pass == 2) {
+                o0 = o;
+                break;
+            }
+            b = o;
+            gb = grad(o);
+            cnn1 = o.czz * t.x * t.x;
+            if(!HEX) pm = add2(p0.p, scl2(halfh, pq0p));
+            qm = add2(p0.q, scl2(halfh, pq0q));
+            u = scl2(o.c, t);
+        }
+        r2.Amp = p0.Amp;
+        r2.Phase = p0.Phase;
+        r2.ntop = p0.ntop;
+        r2.nbot = p0.nbot;
+        r2.c = o0.c;
+        if(w.s.z != s0.z) {   // CurvatureCorrection, 2-D form, depth crossings only
+            const V2<double> gj = sub2(grad(o0), ga);
+            const V2<double> n2 = mk2(-r2.t.y, r2.t.x);
+            const double cnj = dot2(gj, n2), csj = dot2(gj, r2.t);
+            const double rm = fabs(r2.t.y) > 1.0e-100 ? div_rn(r2.t.x, r2.t.y) : r2.t.x / r2.t.y;
+            const double rn = quot_rn(rm * (2.0 * cnj - rm * csj), r2.c, o0.rc);
+            r2.p = sub2(r2.p, scl2(rn, r2.q));
+        }
+        const V3 xe = to_ocean_x(r2.x, org);
+        inside = w.holds(xe);
+        w.boundaries(inside, xe, to_ocean_t(r2.t, org), ctr);
+        return tr ? 1 : br ? 2 : 0;
+    }
+    __device__ __forceinline__ void reflect(int hit, RunCounters *ctr)
+    {
+        RayN old = p0, r;
+        Seg3 s = w.s;
+        Bd3 b = hit == 1 ? w.general(w.top, w.E->btop, w.E->top_ny) : w.general(w.bot, w.E->bbot, w.E->bot_ny);
+        OrgN o = org;
+        reflect_cold_nx(old, r, b, hit == 1, w.E, o, s, ctr);
+        w.set_cell(s);
+        p0 = r;
+        w.eval(to_ocean_x(p0.x, org), to_ocean_t(p0.t, org), o0, ctr);
+        low = p0.Amp < FLTD(0.005);
+    }
+    __device__ __forceinline__ bool stops() const
+    {
+        bool stop = low || small > 50;
+        if(!inside) {
+            const V3 x = to_ocean_x(p0.x, org), t = to_ocean_t(p0.t, org), xs = org.xs;
+            stop = stop || fabs(x.x - xs.x) >= w.E->box_x || fabs(x.y - xs.y) >= w.E->box_y || fabs(x.z) >= w.E->box_z
+                || x.x < minx || x.y < miny || (x.x == minx && t.x < 0.0) || (x.y == miny && t.y < 0.0)
+                || x.x > maxx || x.y > maxy || (x.x == maxx && t.x > 0.0) || (x.y == maxy && t.y > 0.0);
+        }
+        return stop;
+    }
+};
 
 struct CursorN {
     unsigned long long next = 0, end = 0;
@@ -363,20 +531,29 @@ __device__ __forceinline__ void emit_nx(const SegRec<double> &rec, SegRec<double
     for(int k = 0; k < (int)(sizeof(SegRec<double>) / 16); ++k) dst[k] = src[k];
 }
 
-__global__ void __launch_bounds__(64) trace_nx_kernel(const GroupDev *__restrict__ groups, int ngroups,
-                                                      long long job_end, SegRec<double> *segs, unsigned long long cap,
-                                                      RunCounters *ctr, unsigned long long *job_counter)
+// M: 1 when every group of the launch has the hexahedral grid, 2 when every one
+// has a 1-D profile (RayNWalk), 0 for a mixture (general step). Warps take
+// `lanes` consecutive jobs at a time.
+template<int M> __global__ void __launch_bounds__(64) trace_nx_kernel(const GroupDev *__restrict__ groups, int ngroups,
+                                                                      long long job_end, SegRec<double> *segs,
+                                                                      unsigned long long cap, RunCounters *ctr,
+                                                                      unsigned long long *job_counter, int lanes)
 {
+    const int lane = (int)(threadIdx.x & 31);
     for(;;) {
-        const long long job = (long long)atomicAdd(job_counter, 1ull);
-        if(job >= job_end) break;
+        __syncwarp();
+        unsigned long long base = 0;
+        if(lane == 0) base = atomicAdd(job_counter, (unsigned long long)lanes);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if((long long)base >= job_end) break;
+        const long long job = (long long)base + lane;
+        if(lane >= lanes || job >= job_end) continue;
         const GroupDev &G = groups[find_group(groups, ngroups, job)];
         const Env3Dev &E = *G.env3;
         const Job3 J = job_indices3(E, (int)(job - G.job_base));
         if(J.isz >= E.nsz) { run_error(ctr, ERR_RAYINIT); continue; }
         RayStateN st;
         if(!ray_init_nx(E, J, st, ctr)) continue;
-        RayN &p0 = st.p0;
         RayN p1, p2;
         // Init_Influence, 2-D Cartesian geometric (src/influence.hpp:525-644)
         const EnvDev &e = E.e1d;   // the receiver ranges and beam flags of the plane
@@ -386,118 +563,179 @@ __global__ void __launch_bounds__(64) trace_nx_kernel(const GroupDev *__restrict
         const InflEnv ie(e);
         InflState inf;
         inf.phase = 0.0;
-        inf.qOld = p0.q.x;
-        inf.x = p0.x;
-        inf.ir = bsearch_gt(e.rr, e.nrr, p0.x.x);
-        if(p0.t.x < 0.0 && inf.ir > 0) --inf.ir;
+        inf.qOld = st.p0.q.x;
+        inf.x = st.p0.x;
+        inf.ir = bsearch_gt(e.rr, e.nrr, st.p0.x.x);
+        if(st.p0.t.x < 0.0 && inf.ir > 0) --inf.ir;
         inf.r = e.rr[inf.ir];
         int small = 0, is = 0;
         bool overflow = false;
-        unsigned long long nsteps = 0;
+        unsigned int nsteps = 0;
         CursorN cur;
-        for(;;) {
-            if((nsteps & 31) == 0 && __ldcg(&ctr->err_bits) != 0u) break;
-            const bool two = ray_update_nx(st, p1, p2, small, E, ctr);
-            ++nsteps;
+        auto influence = [&](const RayN &a, const RayN &b) {
             SegRec<double> rec;
-            if(infl_prologue(p0, p1, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
+            if(infl_prologue(a, b, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
                 emit_nx(rec, segs, cap, ctr, cur, overflow);
             ++is;
-            if(two) {
-                if(infl_prologue(p1, p2, inf, ie, rcp_q0, ratio1, (int)job, is, rec))
-                    emit_nx(rec, segs, cap, ctr, cur, overflow);
-                p0 = p2;
-                ++is;
+        };
+        RayNWalk<M == 1> ray;
+        if constexpr(M != 0) ray.init(E, st, ctr);
+        for(;;) {
+            if((nsteps & 31) == 0 && __ldcg(&ctr->err_bits) != 0u) break;
+            ++nsteps;
+            if constexpr(M != 0) {
+                const int hit = ray.step(p1, ctr);
+                influence(ray.p0, p1);
+                ray.p0 = p1;
+                if(hit) {
+                    ray.reflect(hit, ctr);
+                    // of no length but at range 0 (trace_kernel)
+                    p2 = ray.p0;
+                    if(p1.x.x == 0.0) influence(p1, p2);
+                    else ++is;
+                }
             } else {
-                p0 = p1;
+                const bool two = ray_update_nx(st, p1, p2, small, E, ctr);
+                influence(st.p0, p1);
+                if(two) influence(p1, p2);
+                st.p0 = two ? p2 : p1;
             }
             if(overflow) {
                 atomicMin(&ctr->overflow_job, (unsigned int)job);
                 run_error(ctr, ERR_SEG_OVERFLOW);
                 break;
             }
-            if(ray_stops_nx(st, small, E)) break;
+            if constexpr(M != 0) {
+                if(ray.stops()) break;
+            } else {
+                if(ray_stops_nx(st, small, E)) break;
+            }
             if(is >= MAXN_STEPS - 3) {
                 run_warn(ctr, WARN_ONERAY_OUTOFMEMORY);
                 break;
             }
         }
         for(; cur.next < cur.end; ++cur.next) segs[cur.next].job = -1;
-        atomicAdd(&ctr->nsteps, nsteps);
+        atomicAdd(&ctr->nsteps, (unsigned long long)nsteps);
     }
 }
 
 // InfluenceGeoCore + ApplyContribution, 2-D Cartesian (src/influence.hpp:
-// 423-473, 897-1024), one thread per (record, receiver depth) over the
-// record's receiver ranges, within the segment's depth window
-// (src/influence.hpp:1285-1292)
-__global__ void __launch_bounds__(128) influence_nx_kernel(const SegRec<double> *__restrict__ segs,
-                                                           unsigned long long cap,
-                                                           const GroupDev *__restrict__ groups, int ngroups,
-                                                           float2 *field, RunCounters *ctr, int nzmax)
+// 423-473, 897-1024). A warp stages 32 records; their (range, depth) items
+// inside the segments' depth windows (src/influence.hpp:1285-1292) are
+// flattened, so that every lane evaluates a receiver. Bound by the FP64 work
+// of the items and the field's 8-byte atomics. With one thread per record and
+// receiver depth, most of them outside the window, and the record read from
+// global memory by each, 12,996 rays x 501 x 101 receivers took 9.6 ms; now 1.5.
+constexpr int WARPSN = 4;
+__global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<double> *__restrict__ segs,
+                                                                   unsigned long long cap,
+                                                                   const GroupDev *__restrict__ groups, int ngroups,
+                                                                   float2 *field, RunCounters *ctr)
 {
+    __shared__ SegRec<double> s_rec[WARPSN][32];
+    __shared__ double s_rcp[WARPSN][32], s_fl[WARPSN][32];
+    __shared__ const Env3Dev *s_env[WARPSN][32];
+    __shared__ long long s_row[WARPSN][32];
+    __shared__ int s_incl[WARPSN][32], s_iz0[WARPSN][32], s_niz[WARPSN][32];
     const unsigned long long nseg = min(__ldcg(&ctr->nseg), cap);
-    const unsigned long long nitems = nseg * (unsigned long long)nzmax;
+    const unsigned long long nchunks = (nseg + 31) / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned int evals = 0;
-    for(unsigned long long it = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; it < nitems;
-        it += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long k = it / (unsigned)nzmax;
-        const int iz = (int)(it - k * (unsigned)nzmax);
-        const SegRec<double> &S = segs[k];
-        if(S.job < 0) continue;
-        const GroupDev &G = groups[find_group(groups, ngroups, S.job)];
-        const Env3Dev &E = *G.env3;
-        if(iz >= E.nrz) continue;
-        const bool gauss = E.gaussian != 0, coherent = E.coherent != 0;
-        const double freq = E.freq0, omega = FLTD(2.0) * BHCB_PI * freq;
-        double sig = S.sigma_seg, fl = 0.0;
-        if(gauss) {   // AdjustSigma (src/influence.hpp:91-100)
-            fl = min(FLTD(0.2) * freq * S.tau1r, BHCB_PI * (S.c0 / freq));
-            sig = max(sig, fl);
+    for(unsigned long long ch = blockIdx.x * (unsigned long long)WARPSN + w; ch < nchunks;
+        ch += (unsigned long long)gridDim.x * WARPSN) {
+        const int nvalid = (int)min(32ull, nseg - ch * 32);
+        {
+            const int words = sizeof(SegRec<double>) / 16;
+            const uint4 *src = reinterpret_cast<const uint4 *>(segs + ch * 32);
+            uint4 *dst = reinterpret_cast<uint4 *>(&s_rec[w][0]);
+            for(int k = lane; k < nvalid * words; k += 32) dst[k] = __ldcs(src + k);
         }
-        const double zr = (double)E.rz[iz];
-        if(fabs(S.tx) > FLTD(0.50001)) {
-            const double rmax = (gauss ? 4.0 : 1.0) * sig;
-            if(zr < S.zlo - rmax || zr > S.zhi + rmax) continue;
+        __syncwarp();
+        int n = 0;
+        const SegRec<double> &M = s_rec[w][lane];
+        if(lane < nvalid && M.job >= 0) {
+            const GroupDev &G = groups[find_group(groups, ngroups, M.job)];
+            const Env3Dev &E = *G.env3;
+            const double freq = E.freq0;
+            double sig = M.sigma_seg, fl = 0.0;
+            if(E.gaussian) {   // AdjustSigma (src/influence.hpp:91-100)
+                fl = min(FLTD(0.2) * freq * M.tau1r, BHCB_PI * (M.c0 / freq));
+                sig = max(sig, fl);
+            }
+            int i0 = 0, i1 = E.nrz;
+            if(fabs(M.tx) > FLTD(0.50001)) {
+                const double rmax = (E.gaussian ? 4.0 : 1.0) * sig;
+                i0 = lower_f(E.rz, E.nrz, M.zlo - rmax);
+                i1 = upper_f(E.rz, E.nrz, M.zhi + rmax);
+            }
+            if(i1 > i0) {
+                n = (M.ir_hi - M.ir_lo + 1) * (i1 - i0);
+                const Job3 J = job_indices3(E, (int)((long long)M.job - G.job_base));
+                s_row[w][lane] = G.field_base
+                    + ((((long long)J.isz * E.nsx + J.isx) * E.nsy + J.isy) * E.ntheta + J.ibeta) * E.nrz * E.nrr;
+                s_env[w][lane] = &E;
+                s_iz0[w][lane] = i0;
+                s_niz[w][lane] = i1 - i0;
+                s_fl[w][lane] = fl;
+                s_rcp[w][lane] = rcp_ulp(M.rlen);
+            }
         }
-        const Job3 J = job_indices3(E, (int)((long long)S.job - G.job_base));
-        float2 *row = field + G.field_base
-            + ((((long long)J.isz * E.nsx + J.isx) * E.nsy + J.isy) * E.ntheta + J.ibeta) * E.nrz * E.nrr
-            + (long long)iz * E.nrr;
-        const double dz = zr - S.x0z;
-        for(int ir = S.ir_lo; ir <= S.ir_hi; ++ir) {
-            const double dr = E.rr[ir] - S.x0r;
-            const double s = (dr * S.tx + dz * S.tz) / S.rlen;
+        int incl = n;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if(lane >= o) incl += v;
+        }
+        s_incl[w][lane] = incl;
+        __syncwarp();
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        for(int it = lane; it < total; it += 32) {
+            int lo = 0, hi = 31;   // first record j with incl[j] > it
+            while(lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if(s_incl[w][mid] > it) hi = mid; else lo = mid + 1;
+            }
+            const int j = lo, local = it - (j ? s_incl[w][j - 1] : 0);
+            const int niz = s_niz[w][j], col = local / niz, iz = s_iz0[w][j] + local - col * niz;
+            const SegRec<double> &S = s_rec[w][j];
+            const Env3Dev &E = *s_env[w][j];
+            const bool gauss = E.gaussian != 0, coherent = E.coherent != 0;
+            const int ir = S.ir_lo + col;
+            const double dz = (double)E.rz[iz] - S.x0z, dr = E.rr[ir] - S.x0r;
+            const double s = quot_rn(dr * S.tx + dz * S.tz, S.rlen, s_rcp[w][j]);
             const double n1 = fabs(dz * S.tx - dr * S.tz);
             const double qF = S.q0 + s * S.dq;
             double sigma = fabs(qF * S.rcp_q0);
             const double sig0 = sigma;
-            if(gauss) sigma = max(sigma, fl);
+            if(gauss) sigma = max(sigma, s_fl[w][j]);
             if(n1 >= (gauss ? 4.0 : 1.0) * sigma) continue;
             const double cnst = S.cnst_num / sqrt(fabs(qF));
-            const double w = gauss ? exp(FLTD(-0.5) * (n1 / sigma) * (n1 / sigma)) * (sig0 / sigma)
-                                   : (sigma - n1) / sigma;
+            const double wgt = gauss ? exp(FLTD(-0.5) * (n1 / sigma) * (n1 / sigma)) * (sig0 / sigma)
+                                     : (sigma - n1) / sigma;
             const bool caustic = (qF <= 0.0 && S.q0 > 0.0) || (qF >= 0.0 && S.q0 < 0.0);
             const double ph = caustic ? S.phase_b : S.phase_a;
+            const double omega = FLTD(2.0) * BHCB_PI * E.freq0;
             const double di = S.tau0i + s * S.dtaui;
             float2 v;
             if(coherent) {
-                const double amp = cnst * w * exp(omega * di);
+                const double amp = cnst * wgt * exp(omega * di);
                 double sn, cs;
                 sincos(reduce_2pi(omega * (S.tau0r + s * S.dtaur) - ph), &sn, &cs);
                 v = make_float2((float)(amp * cs), (float)(-amp * sn));
             } else {
                 double vv = cnst * exp(omega * di);
-                vv = vv * vv * w;
+                vv = vv * vv * wgt;
                 if(gauss) vv *= sqrt(FLTD(2.0) * BHCB_PI);
                 v = make_float2((float)vv, 0.f);
             }
-            atomicAdd(row + ir, v);
+            atomicAdd(field + s_row[w][j] + (long long)iz * E.nrr + ir, v);
             ++evals;
         }
+        __syncwarp();
     }
     for(int o = 16; o > 0; o >>= 1) evals += __shfl_xor_sync(0xffffffffu, evals, o);
-    if((threadIdx.x & 31) == 0 && evals) atomicAdd(&ctr->nevals, (unsigned long long)evals);
+    if(lane == 0 && evals) atomicAdd(&ctr->nevals, (unsigned long long)evals);
 }
 
 // Arrivals, Nx2D: the contributions of influence_nx_kernel as arrival
@@ -717,11 +955,15 @@ cudaError_t launch_rays_nx(const GroupDev *groups, int ngroups, const long long 
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace_nx(const GroupDev *groups, int ngroups, long long job_end, void *segs,
-                            unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, int grid,
-                            cudaStream_t st)
+cudaError_t launch_trace_nx(const GroupDev *groups, int ngroups, long long njobs, long long job_end, void *segs,
+                            unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, int sm_count,
+                            int kind, cudaStream_t st)
 {
-    trace_nx_kernel<<<grid, 64, 0, st>>>(groups, ngroups, job_end, (SegRec<double> *)segs, cap, ctr, job_counter);
+    const int lanes = lanes3(njobs, sm_count);
+    const long long warps = (njobs + lanes - 1) / lanes;
+    const int grid = (int)std::max(1LL, std::min<long long>((warps + 1) / 2, (long long)sm_count * 16));
+    auto k = kind == 1 ? trace_nx_kernel<1> : kind == 2 ? trace_nx_kernel<2> : trace_nx_kernel<0>;
+    k<<<grid, 64, 0, st>>>(groups, ngroups, job_end, (SegRec<double> *)segs, cap, ctr, job_counter, lanes);
     return cudaGetLastError();
 }
 
@@ -742,10 +984,9 @@ cudaError_t launch_arr_gather_nx(const void *segs, unsigned long long nseg, cons
 }
 
 cudaError_t launch_influence_nx(const void *segs, unsigned long long cap, const GroupDev *groups, int ngroups,
-                                float2 *field, RunCounters *ctr, int nzmax, int grid, cudaStream_t st)
+                                float2 *field, RunCounters *ctr, int grid, cudaStream_t st)
 {
-    if(nzmax < 1) nzmax = 1;
-    influence_nx_kernel<<<grid, 128, 0, st>>>((const SegRec<double> *)segs, cap, groups, ngroups, field, ctr, nzmax);
+    influence_nx_kernel<<<grid, 32 * WARPSN, 0, st>>>((const SegRec<double> *)segs, cap, groups, ngroups, field, ctr);
     return cudaGetLastError();
 }
 

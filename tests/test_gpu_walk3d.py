@@ -64,6 +64,9 @@ CASES.update({
     "hex_on_face": dict(ssp_opt="HVW", hexa=True, sx=[1.5], sy=[1.5], sz=[400.0], bty=bowl(), box_km=(3.4, 3.4)),
     "hex_hat_incoherent": dict(ssp_opt="HVW", hexa=True, bty=bowl(), run_type="IG   3"),
 })
+# the same ocean as N x 2-D rays (trace_nx_kernel); not the displaced sources, whose planes leave the grid
+CASES.update({"nx2d_" + k: dict(v, run_type=v.get("run_type", "CB   3").replace("3", "2")) for k, v in CASES.items()
+              if k not in ("off_centre", "hex_on_face")})
 
 
 def run(roots):
@@ -77,7 +80,11 @@ def run(roots):
 
 @pytest.mark.parametrize("case", sorted(CASES))
 def test_alone_equals_general_step(case, tmp_path):
-    other = dict() if case.startswith("hex") else dict(ssp_opt="HVW", hexa=True)
+    other = dict() if "hex" in case else dict(ssp_opt="HVW", hexa=True)
+    if CASES[case].get("run_type", "")[-1:] == "2":
+        other["run_type"] = "CB   2"
+    if "IG" in CASES[case].get("run_type", ""):   # a batch has one beam type and coherence
+        other["run_type"] = CASES[case]["run_type"]
     a = write_files(files(**CASES[case]), os.path.join(str(tmp_path), "a"))
     b = write_files(files(alpha=(5, -10.0, 10.0), **other), os.path.join(str(tmp_path), "b"))
     (fa,), sa, ea = run([a])
