@@ -49,12 +49,12 @@ cudaError_t radix_sort_pairs(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uns
 cudaError_t launch_arr_replay(const uint64_t *, const uint32_t *, const ArrCand *, unsigned long long,
                               const GroupDev *, int, const double *, long long, int, int, int, int32_t *,
                               ArrivalRec *, int, cudaStream_t, bool);
-cudaError_t launch_rays(const GroupDev *, int, const long long *, const int *, int, const long long *, double2 *, int *,
-                        int *, RunCounters *, bool, int, cudaStream_t);
+cudaError_t launch_rays(const GroupDev *, int, const long long *, const int *, int, const long long *, const int *,
+                        double2 *, int *, int *, RunCounters *, bool, int, cudaStream_t);
 cudaError_t launch_eigen_emit(const uint32_t *, const ArrCand *, unsigned long long, EigenHitRec *, int32_t *, int,
                               const uint64_t *, int, cudaStream_t);
-cudaError_t launch_trace_x(const GroupDev *, int, long long, XSeg *, unsigned long long, RunCounters *,
-                           unsigned long long *, int, int, int, cudaStream_t);
+cudaError_t launch_trace_x(const GroupDev *, int, int, XSeg *, unsigned long long, RunCounters *,
+                           unsigned long long *, int, bool, int, cudaStream_t);
 cudaError_t launch_influence_x(const XSeg *, unsigned long long, const GroupDev *, int, const double *, float2 *,
                                RunCounters *, int, int, int, cudaStream_t);
 cudaError_t launch_scale_x(const float2 *, float2 *, const GroupDev *, int, const double *, RunCounters *, int,
@@ -386,6 +386,14 @@ void plan_lanes(bhcb_ctx *c)
     CK(cudaMemcpyAsync(c->groups_d.p, c->groups_h.data(), ng * sizeof(GroupDev), cudaMemcpyHostToDevice, c->stream));
 }
 
+// every group of [g0, g1) has packed segments
+bool all_seg(const bhcb_ctx *c, int g0, int g1)
+{
+    for(int g = g0; g < g1; ++g)
+        if(!c->envdev_h[g].has_seg) return false;
+    return true;
+}
+
 // Packed segments of a profile of type C, S or P; empty for other types, for
 // complex sound speeds and for fewer than two nodes.
 std::vector<SspSeg> pack_segments(const EnvTables &T)
@@ -645,9 +653,8 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
     RunCounters *ctr = (RunCounters *)c->counters.p;
     CK(cudaMemsetAsync(&ctr->overflow_job, 0xff, sizeof(ctr->overflow_job), c->stream));
     unsigned long long *jobc = (unsigned long long *)((uint8_t *)c->counters.p + sizeof(RunCounters));
-    // the x kinds' trace counts rays, the Cartesian one blocks of rays
-    const long long first = c->xkind ? job0 : (long long)c->groups_h[g0].blk_base;
-    if(first) CK(launch_set_counter(jobc, (unsigned long long)first, c->stream));
+    const int blk0 = c->groups_h[g0].blk_base, blk1 = g1 < ngall ? c->groups_h[g1].blk_base : c->nblocks;
+    if(blk0) CK(launch_set_counter(jobc, (unsigned long long)blk0, c->stream));
     if(clear) {
         const int64_t a0 = c->groups_h[g0].acc_base;
         const int64_t a1 = g1 < ngall ? c->groups_h[g1].acc_base : c->total_acc;
@@ -659,9 +666,9 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
         // kind's influence prologue, then its influence kernel and scaling
         const GroupDev *Gx = (const GroupDev *)c->groups_d.p + g0;
         const int ngx = g1 - g0;
-        long long xgrid = std::min<long long>((job1 - job0 + 63) / 64, (long long)c->sm_count * 16);
-        CK(launch_trace_x(Gx, ngx, job1, (XSeg *)c->segs.p, c->seg_cap, ctr, jobc, c->xkind, (int)std::max(1LL, xgrid),
-                          64, c->stream));
+        const int xgrid = std::max(1, std::min((blk1 - blk0 + 1) / 2, c->sm_count * 16));
+        CK(launch_trace_x(Gx, ngx, blk1, (XSeg *)c->segs.p, c->seg_cap, ctr, jobc, c->xkind, all_seg(c, g0, g1), xgrid,
+                          c->stream));
         CK(record_event(c, 1, c->stream));
         if(c->mode != MODE_TL) return;   // arrivals / hits: run_arrivals after the trace
         c->last_overlapped = false;
@@ -675,7 +682,6 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
         CK(record_event(c, 3, c->stream));
         return;
     }
-    const int blk0 = c->groups_h[g0].blk_base, blk1 = g1 < ngall ? c->groups_h[g1].blk_base : c->nblocks;
     int tblock = c->trace_block;
     unsigned int stage_bytes = 0;   // tables of the launched groups that fit the staging budget
     for(int g = g0; g < g1; ++g) {
@@ -950,9 +956,10 @@ int group_of_field(const bhcb_ctx *c, int fi)
     throw std::runtime_error("field has no trace group");
 }
 
-// Trajectories of R.jobs (limits as for the ray kernel): a count pass sizes
-// the point buffer exactly, a second pass of the same deterministic trace
-// writes the points; both passes read the context's prepared tables.
+// Trajectories of R.jobs (limits as for the ray kernel). A ray with a limit has
+// at most limit + 3 points, so eigenrays are traced once, into as much room (a pass of two saved), and
+// packed as they leave; rays without one are counted by a pass of their own,
+// which sizes the buffer of a second pass of the same deterministic trace.
 void trace_rays(bhcb_ctx *c, RaySet &R)
 {
     const int n = (int)R.jobs.size();
@@ -962,22 +969,42 @@ void trace_rays(bhcb_ctx *c, RaySet &R)
     R.rz.clear();
     R.valid = true;
     if(n == 0) return;
-    DevBuf jobs_d, lim_d, npts_d, bnc_d, off_d, pts_d;
+    std::vector<int> room(n);
+    long long tot = 0;
+    bool once = true;
+    for(int i = 0; i < n; ++i) {
+        once = once && R.limits[i] >= 0;
+        room[i] = std::max(R.limits[i], 0) + 3;
+        R.off[i] = tot;
+        tot += room[i];
+    }
+    once = once && (size_t)tot * sizeof(double2) <= c->max_memory;
+    DevBuf jobs_d, lim_d, npts_d, bnc_d, off_d, room_d, pts_d;
     jobs_d.ensure(n * sizeof(long long));
     lim_d.ensure(n * sizeof(int));
     npts_d.ensure(n * sizeof(int));
     bnc_d.ensure(2 * (size_t)n * sizeof(int));
     off_d.ensure(n * sizeof(long long));
-    auto release = [&]() { for(DevBuf *b : {&jobs_d, &lim_d, &npts_d, &bnc_d, &off_d, &pts_d}) b->release(); };
+    room_d.ensure(n * sizeof(int));
+    auto release = [&]() { for(DevBuf *b : {&jobs_d, &lim_d, &npts_d, &bnc_d, &off_d, &room_d, &pts_d}) b->release(); };
     try {
         CK(cudaMemcpyAsync(jobs_d.p, R.jobs.data(), n * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(lim_d.p, R.limits.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemsetAsync(c->counters.p, 0, sizeof(RunCounters), c->stream));
         RunCounters *ctr = (RunCounters *)c->counters.p;
-        const GroupDev *G = (const GroupDev *)c->groups_d.p;
         const int ng = (int)c->groups_h.size();
-        CK(launch_rays(G, ng, (const long long *)jobs_d.p, (const int *)lim_d.p, n, nullptr, nullptr,
-                       (int *)npts_d.p, (int *)bnc_d.p, ctr, true, c->sm_count, c->stream));
+        auto trace = [&](bool write, bool count) {
+            if(write) {
+                pts_d.ensure(std::max<long long>(tot, 1) * sizeof(double2));
+                CK(cudaMemcpyAsync(off_d.p, R.off.data(), n * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+                CK(cudaMemcpyAsync(room_d.p, room.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+            }
+            CK(launch_rays((const GroupDev *)c->groups_d.p, ng, (const long long *)jobs_d.p, (const int *)lim_d.p, n,
+                           (const long long *)off_d.p, (const int *)room_d.p,
+                           write ? (double2 *)pts_d.p : nullptr, count ? (int *)npts_d.p : nullptr,
+                           (int *)bnc_d.p, ctr, all_seg(c, 0, ng), c->sm_count, c->stream));
+        };
+        trace(once, true);
         CK(cudaMemcpyAsync(R.npts.data(), npts_d.p, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaMemcpyAsync(R.bnc.data(), bnc_d.p, 2 * (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         RunCounters rc{};
@@ -987,20 +1014,30 @@ void trace_rays(bhcb_ctx *c, RaySet &R)
             c->err_bits = rc.err_bits;
             throw std::runtime_error("tracer error while tracing rays");
         }
-        long long tot = 0;
-        for(int i = 0; i < n; ++i) {
-            R.off[i] = tot;
-            tot += R.npts[i];
+        if(!once) {
+            tot = 0;
+            for(int i = 0; i < n; ++i) {
+                R.off[i] = tot;
+                room[i] = R.npts[i];
+                tot += R.npts[i];
+            }
+            if((size_t)tot * sizeof(double2) > c->max_memory) throw MemError("ray points exceed max_memory");
+            trace(true, false);
         }
-        if((size_t)tot * sizeof(double2) > c->max_memory) throw MemError("ray points exceed max_memory");
-        pts_d.ensure(std::max<long long>(tot, 1) * sizeof(double2));
-        CK(cudaMemcpyAsync(off_d.p, R.off.data(), n * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
-        CK(launch_rays(G, ng, (const long long *)jobs_d.p, (const int *)lim_d.p, n, (const long long *)off_d.p,
-                       (double2 *)pts_d.p, (int *)npts_d.p, (int *)bnc_d.p, ctr, false, c->sm_count, c->stream));
         R.rz.resize(2 * (size_t)tot);
         if(tot)
             CK(cudaMemcpyAsync(R.rz.data(), pts_d.p, tot * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
+        if(once) {
+            long long to = 0;
+            for(int i = 0; i < n; ++i) {
+                if(to != R.off[i])
+                    std::memmove(&R.rz[2 * (size_t)to], &R.rz[2 * (size_t)R.off[i]], R.npts[i] * sizeof(double2));
+                R.off[i] = to;
+                to += R.npts[i];
+            }
+            R.rz.resize(2 * (size_t)to);
+        }
         c->warn_bits |= rc.warn_bits;
     } catch(...) {
         release();

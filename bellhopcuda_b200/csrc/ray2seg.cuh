@@ -135,7 +135,11 @@ __device__ __forceinline__ BdryPos reflect_rare(const EnvDev *e, BdryPos b, bool
     return b;
 }
 
+// K: the profile type, or SSP_ANY for the one of the environment (kernels whose
+// prologues differ by beam type, which would otherwise be compiled three times)
+constexpr int SSP_ANY = -1;
 template<int K> struct Ray2Seg {
+    int kind;
     const EnvDev *e;
     const SspSeg *tab;
     RayPt<double> p0;
@@ -159,7 +163,7 @@ template<int K> struct Ray2Seg {
         const double2 *r = reinterpret_cast<const double2 *>(tab + i);
         const double2 a = r[0], b = r[1];
         z0 = a.x; z1 = a.y; k0 = b.x; k1 = b.y;
-        if(K != SSP_CLINEAR) {
+        if((K < 0 ? kind : K) != SSP_CLINEAR) {
             const double2 d = r[2];
             k2 = d.x; k3 = d.y;
         }
@@ -180,11 +184,12 @@ template<int K> struct Ray2Seg {
     {
         find_seg(y, ty >= 0.0);
         const double h = y - z0;
-        if(K == SSP_CLINEAR) {
+        const int k = K < 0 ? kind : K;
+        if(k == SSP_CLINEAR) {
             c_ = k0 + h * k1;
             g_ = k1;
             czz_ = 0.0;
-        } else if(K == SSP_CUBIC) {
+        } else if(k == SSP_CUBIC) {
             const double half = 0.5, sixth = (double)(1.0f / 6.0f);
             c_ = k0 + h * (k1 + h * (half * k2 + sixth * h * k3));
             g_ = k1 + h * (k2 + h * half * k3);
@@ -218,6 +223,7 @@ template<int K> struct Ray2Seg {
     __device__ __forceinline__ void init(const RayState2<double> &st, const EnvDev &env)
     {
         e = &env;
+        kind = env.ssp_type;
         tab = env.segtab;
         p0 = st.p0;
         deltas = env.deltas;
