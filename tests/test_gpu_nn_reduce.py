@@ -1,0 +1,52 @@
+"""The surrogate's reductions against float64: bias gradients (column sums of a
+bf16 matrix) and the squared-error loss with its gradient, at the edges of their
+splits (64 columns a block, 32 rows a turn, a cluster from 4096 rows on), for
+odd widths and unaligned bases.
+
+A column sum adds at most M / 32 + 40 terms one after another in FP32, each
+addition within 2^-24 of a partial sum that is at most sum |dy|. The loss is
+FP64: n * 2^-53 of it. The gradient is one bf16 rounding of scale * 2 d."""
+import ctypes as C
+
+import pytest
+
+import bellhopcuda_b200 as B
+
+pytestmark = pytest.mark.gpu
+
+
+def ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def stream():
+    import torch
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("M", [1, 31, 33, 256, 4095, 4096, 32768])
+@pytest.mark.parametrize("N,shift", [(1, 0), (8, 0), (63, 0), (64, 1), (66, 0), (512, 0)])
+def test_colsum(M, N, shift):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    dy = torch.randn(M * N + shift, device="cuda", generator=g).bfloat16()[shift:].view(M, N)
+    db = torch.full((N + 1,), 7.0, device="cuda")
+    assert B.load_library().bhcb_nn_colsum(ptr(dy), M, N, ptr(db), stream()) == 0
+    d = dy.double()
+    bound = (M / 32 + 40) * 2.0 ** -24 * d.abs().sum(0)
+    assert bool(((db[:N].double() - d.sum(0)).abs() <= bound).all()) and db[N].item() == 7.0
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (3, 0), (255, 1), (1024, 0), (1027, 0), (2097155, 0), (300000, 1)])
+def test_mse(n, shift):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    p, t = (torch.randn(n + shift, device="cuda", generator=g)[shift:] for _ in range(2))
+    grad = torch.zeros(n + 1, device="cuda", dtype=torch.bfloat16)
+    loss = torch.full((1,), 0.25, device="cuda", dtype=torch.float64)
+    assert B.load_library().bhcb_nn_mse(ptr(p), ptr(t), n, 0.37, ptr(grad), ptr(loss), stream()) == 0
+    d = p - t
+    ref = 0.25 + (d.double() ** 2).sum().item()
+    assert abs(loss.item() - ref) <= n * 2.0 ** -53 * ref
+    s = torch.tensor(0.37, device="cuda") * 2.0
+    assert torch.equal(grad[:n], (s * d).bfloat16()) and grad[n].item() == 0.0
