@@ -149,6 +149,7 @@ SIGNATURES = [
     ("bhcb_graph_destroy", None, [C.c_void_p]),
     ("bhcb_nn_gemm", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    ("bhcb_nn_gemm_t", C.c_int, [C.c_void_p] * 3 + [C.c_int32] * 6 + [C.c_void_p] * 5),
     ("bhcb_nn_status", C.c_int, [C.POINTER(C.c_int32), C.c_int32]),
     ("bhcb_nn_tl_db", C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float, C.c_void_p]),
     ("bhcb_nn_transpose", C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p]),

@@ -2,6 +2,11 @@
 //
 //   C[M, N] = epilogue(A[M, K] * B[N, K]^T)      A, B row-major bf16 (K-major)
 //
+// Either operand may instead be stored as its transpose, [K, M] or [K, N]
+// (MN-major): the tensor cores read both layouts, so the backward products need
+// no transposed copies. With A transposed, its column sums over K (the bias
+// gradient of a weight-gradient product) come from CTAs of the same launch.
+//
 // One CTA per 128 x 128 or 128 x 32 output tile, 128 threads:
 //   warp 0 lane 0  TMA producer: 64-deep bf16 tiles of A and B into a ring of
 //                  stages (128-byte swizzle), completion on the stage's "full"
@@ -37,7 +42,7 @@ constexpr int TILE_A = BM * BK * 2;   // 16 KiB
 // Two tile widths. 128 columns, 3 CTAs per SM, for outputs of many tiles; 32
 // columns, one CTA per SM with a ring of 160 KiB, for outputs of few: four times
 // the CTAs, each bound by its SM's port from L2 (160 rows of 128 bytes per 64 of
-// K; 512 x 512 x 32768: 72 us, 145 GB/s per SM). Splitting K would fill the chip
+// K; 512 x 512 x 32768: 82 us, 128 GB/s per SM). Splitting K would fill the chip
 // further, but the accumulator truncates, so at K = 32768 its sum depends on the
 // order by 1e-4.
 template<int BN> struct Tile {
@@ -46,8 +51,10 @@ template<int BN> struct Tile {
     static constexpr int CTAS = BN == 128 ? 3 : 1;
     static constexpr int TILE_B = BN * BK * 2;
     static constexpr int SMEM_BYTES = STAGES * KS * (TILE_A + TILE_B) + 1024 + 256;
+    static constexpr int SUM_STAGES = BN == 128 ? 4 : 8;   // of 128 rows x 64 columns (column_sums)
     // instruction descriptor: FP32 accumulate (bit 4), A and B BF16 (bits 7, 10),
-    // both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+    // transposed A and B (bits 15, 16, set at run time), N >> 3 at bit 17, M >> 4
+    // at bit 24
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17)
         | ((uint32_t)(BM >> 4) << 24);
 };
@@ -84,6 +91,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
         if(mbar_try_wait(bar, parity)) return true;
     return false;
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)
 {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
@@ -91,15 +102,17 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
                  : "memory");
 }
-// shared-memory matrix descriptor of a K-major tile with 128-byte rows in the
-// 128-byte swizzle (8-row groups 1024 bytes apart)
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr)
+// shared-memory matrix descriptor. K-major: 128-byte rows (64 K) in the 128-byte
+// swizzle, groups of 8 rows `sbo` bytes apart. MN-major: rows of 128 (or, for a
+// 32-wide tile, 64) bytes of M or N, one per K, groups of 8 K `sbo` bytes apart,
+// the next 64 of M or N `lbo` bytes on.
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo, bool sw64)
 {
     uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1 << 16;             // leading byte offset (unused when swizzled)
-    d |= (uint64_t)(1024 >> 4) << 32;   // stride byte offset
-    d |= (uint64_t)1 << 46;             // descriptor version
-    d |= (uint64_t)2 << 61;             // 128-byte swizzle
+    d |= (uint64_t)(lbo >> 4) << 16;
+    d |= (uint64_t)(sbo >> 4) << 32;
+    d |= (uint64_t)1 << 46;                  // descriptor version
+    d |= (uint64_t)(sw64 ? 4 : 2) << 61;     // 64- or 128-byte swizzle
     return d;
 }
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
@@ -164,33 +177,122 @@ __device__ __forceinline__ uint4 pack_bf16(const float *x)
     return *reinterpret_cast<const uint4 *>(h);
 }
 
-// vec: rows of C, aux_in and aux_out, and bias, may be accessed 16 bytes at a time
+// db[c] = sum over the K rows of columns [c0, c0 + 64) of A, stored [K][M]: the
+// rows one after another in FP32, as one thread per column would add them (the
+// weights' later roundings hang on the last bits of these sums). TMA fills the
+// ring; two warps add 32 columns each, sixteen rows read ahead of the additions,
+// 7 cycles a row in all: 32768 rows in 120 us beside a product of 75
+// (a column per thread from global memory took 1915).
+template<int BN>
+__device__ __forceinline__ void column_sums(uint8_t *ring, uint64_t *full, uint64_t *empty, const CUtensorMap *tmA,
+                                            int c0, int M, int K, float *db, int *s_fail)
+{
+    constexpr int NS = Tile<BN>::SUM_STAGES, BYTES = 128 * 128;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nk = (K + 127) / 128;
+    if(warp == 0 && lane == 0) {
+        for(int kb = 0; kb < nk; ++kb) {
+            const int s = kb % NS;
+            if(kb >= NS && !mbar_wait(&empty[s], (kb / NS - 1) & 1)) {
+                *s_fail = 1;
+                break;
+            }
+            mbar_expect_tx(&full[s], BYTES);
+            tma_load_2d(ring + s * BYTES, tmA, &full[s], c0, kb * 128);
+            tma_load_2d(ring + s * BYTES + BYTES / 2, tmA, &full[s], c0, kb * 128 + 64);
+        }
+    } else if(warp >= 2) {
+        const int col = (warp - 2) * 32 + lane;
+        uint32_t at[8];   // of this column in row r: 16-byte chunk c of the row lies at c ^ (r & 7)
+#pragma unroll
+        for(int r = 0; r < 8; ++r) at[r] = (uint32_t)(r * 128 + (((col >> 3) ^ r) << 4) + (col & 7) * 2);
+        float sum = 0.0f;
+        uint32_t v[2][16];
+        auto read = [&](int stage, int g, uint32_t *o) {
+            const uint8_t *t = ring + stage * BYTES + g * 2048;
+#pragma unroll
+            for(int r = 0; r < 16; ++r)
+                o[r] = *reinterpret_cast<const unsigned short *>(t + (r >> 3) * 1024 + at[r & 7]);
+        };
+        int s = 0;
+        uint32_t parity = 0;
+        bool ok = mbar_wait(&full[0], 0);
+        if(ok) read(0, 0, v[0]);
+        for(int kb = 0; ok && kb < nk; ++kb) {
+            const int next = s + 1 == NS ? 0 : s + 1;
+            if(next == 0) parity ^= 1;
+#pragma unroll
+            for(int g = 0; g < 8; ++g) {
+                if(g < 7) {
+                    read(s, g + 1, v[(g + 1) & 1]);
+                } else if(kb + 1 < nk) {
+                    ok = mbar_wait(&full[next], parity);
+                    if(ok) read(next, 0, v[0]);
+                }
+#pragma unroll
+                for(int r = 0; r < 16; ++r) sum += __uint_as_float(v[g & 1][r] << 16);   // rows past K are +0
+            }
+            __syncwarp();
+            if(lane == 0) mbar_arrive(&empty[s]);
+            s = next;
+        }
+        if(!ok) {
+            *s_fail = 1;
+            return;
+        }
+        if(c0 + col < M) db[c0 + col] = sum;
+    }
+}
+
+// vec: rows of C, aux_in and aux_out, and bias, may be accessed 16 bytes at a time.
+// a_mn, b_mn: A, B stored [K][M], [K][N]. colsum (a_mn only): blocks of
+// blockIdx.z 0 are its CTAs, the product's are the next layer.
 template<int EPI, int BN>
 __global__ void __launch_bounds__(128, Tile<BN>::CTAS)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                    int K, void *C, const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ aux_in,
-                   __nv_bfloat16 *aux_out, int vec)
+                   __nv_bfloat16 *aux_out, int vec, int a_mn, int b_mn, float *colsum)
 {
     constexpr int STAGES = Tile<BN>::STAGES, KS = Tile<BN>::KS, TILE_B = Tile<BN>::TILE_B;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    // (an offset, so that accesses stay shared-memory ones)
+    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t *sA = smem;
     uint8_t *sB = smem + STAGES * KS * TILE_A;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * KS * (TILE_A + TILE_B));
-    uint64_t *empty = full + STAGES;
-    uint64_t *done = empty + STAGES;
+    constexpr int BARS = Tile<BN>::SUM_STAGES > STAGES ? Tile<BN>::SUM_STAGES : STAGES;
+    uint64_t *empty = full + BARS;
+    uint64_t *done = empty + BARS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     __shared__ int s_fail;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if(colsum && blockIdx.z == 0) {
+        const int c0 = 64 * ((int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x);
+        if(c0 >= M) return;
+        if(threadIdx.x == 0) {
+            s_fail = 0;
+            for(int s = 0; s < Tile<BN>::SUM_STAGES; ++s) {
+                mbar_init(&full[s], 1);
+                mbar_init(&empty[s], 2);
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncthreads();
+        column_sums<BN>(smem, full, empty, &tmA, c0, M, K, colsum, &s_fail);
+        __syncthreads();
+        if(threadIdx.x == 0 && s_fail) atomicExch(&g_nn_error, 1);
+        return;
+    }
     // Tile order: the launch order walks groups of GROUP_M tile rows, a column
     // of GROUP_M tiles at a time, so the CTAs resident together share GROUP_M
     // panels of A and a band of B panels that fit in L2 (instead of every B
     // panel against a few A rows).
     int m_t, n_t;
     {
-        const int num_m = (int)gridDim.y, num_n = (int)gridDim.x;
-        const int t = (int)blockIdx.y * num_n + (int)blockIdx.x;
+        const int num_m = (int)gridDim.y, num_n = (N + BN - 1) / BN;
+        const int t = (int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x;
+        if(t >= num_m * num_n) return;   // a layer widened for the column sums
         const int per_group = GROUP_M * num_n;
         const int first_m = (t / per_group) * GROUP_M;
         const int gsz = min(num_m - first_m, GROUP_M);
@@ -230,8 +332,20 @@ __global__ void __launch_bounds__(128, Tile<BN>::CTAS)
             mbar_expect_tx(&full[s], KS * (TILE_A + TILE_B));
 #pragma unroll
             for(int j = 0; j < KS; ++j) {
-                tma_load_2d(sA + (s * KS + j) * TILE_A, &tmA, &full[s], (kb * KS + j) * BK, m0);
-                tma_load_2d(sB + (s * KS + j) * TILE_B, &tmB, &full[s], (kb * KS + j) * BK, n0);
+                const int k0 = (kb * KS + j) * BK;
+                uint8_t *a = sA + (s * KS + j) * TILE_A, *b = sB + (s * KS + j) * TILE_B;
+                if(a_mn) {
+                    tma_load_2d(a, &tmA, &full[s], m0, k0);
+                    tma_load_2d(a + TILE_A / 2, &tmA, &full[s], m0 + 64, k0);
+                } else {
+                    tma_load_2d(a, &tmA, &full[s], k0, m0);
+                }
+                if(b_mn) {
+                    tma_load_2d(b, &tmB, &full[s], n0, k0);
+                    if(BN == 128) tma_load_2d(b + TILE_B / 2, &tmB, &full[s], n0 + 64, k0);
+                } else {
+                    tma_load_2d(b, &tmB, &full[s], k0, n0);
+                }
             }
         }
     } else if(warp == 1) {
@@ -241,7 +355,13 @@ __global__ void __launch_bounds__(128, Tile<BN>::CTAS)
         // K block of 64 whatever the tile, now 250
         bool ok = true;
         const uint32_t issue = elect_one();
-        const uint64_t dA = sw128_desc(smem_u32(sA)), dB = sw128_desc(smem_u32(sB));
+        const uint64_t dA = make_desc(smem_u32(sA), a_mn ? TILE_A / 2 : 16, 1024, false);
+        const uint64_t dB = b_mn && BN == 32 ? make_desc(smem_u32(sB), 16, 512, true)
+                                             : make_desc(smem_u32(sB), b_mn ? TILE_B / 2 : 16, 1024, false);
+        // a K step of 16, in the descriptors' units of 16 bytes: 32 bytes along a
+        // K-major row, or 16 rows
+        const int ka = a_mn ? 128 : 2, kbs = b_mn ? (BN == 32 ? 64 : 128) : 2;
+        const uint32_t idesc = Tile<BN>::IDESC | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16);
         int s = 0;
         uint32_t parity = 0;
         for(int kb = 0; kb < nk; ++kb) {
@@ -250,14 +370,12 @@ __global__ void __launch_bounds__(128, Tile<BN>::CTAS)
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // descriptors count in 16 bytes: 32 along a swizzled row per K step of 16
             const uint64_t a0 = dA + (uint64_t)(s * KS * (TILE_A >> 4)), b0 = dB + (uint64_t)(s * KS * (TILE_B >> 4));
             if(issue) {
 #pragma unroll
                 for(int k = 0; k < KS * 4; ++k)
-                    umma_bf16(tmem, a0 + (k & 3) * 2 + (k >> 2) * (TILE_A >> 4),
-                              b0 + (k & 3) * 2 + (k >> 2) * (TILE_B >> 4), Tile<BN>::IDESC,
-                              (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_bf16(tmem, a0 + (k & 3) * ka + (k >> 2) * (TILE_A >> 4),
+                              b0 + (k & 3) * kbs + (k >> 2) * (TILE_B >> 4), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 umma_commit(&empty[s]);
             }
             __syncwarp();
@@ -385,24 +503,33 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-// rows x K row-major bf16, boxes of 64 columns x box_rows rows, 128-byte swizzle,
-// out-of-range elements read as zero
-bool make_map(CUtensorMap *map, const void *ptr, int rows, int K, int box_rows)
+// rows x cols row-major bf16, boxes of box_rows x box_cols, swizzled by their
+// width, out-of-range elements read as zero
+bool make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_rows, int box_cols)
 {
     EncodeTiledFn enc = encode_fn();
     if(!enc) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+               CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template<int EPI, int BN>
-void launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K, void *C, const float *bias,
-                 const __nv_bfloat16 *ai, __nv_bfloat16 *ao, int vec, cudaStream_t st)
+struct GemmArgs {
+    CUtensorMap ma, mb;
+    int M, N, K;
+    void *C;
+    const float *bias;
+    const __nv_bfloat16 *aux_in;
+    __nv_bfloat16 *aux_out;
+    int vec, a_mn, b_mn;
+    float *colsum;
+};
+
+template<int EPI, int BN> void launch_gemm(const GemmArgs &g, cudaStream_t st)
 {
     static bool done = false;
     if(!done) {
@@ -410,23 +537,24 @@ void launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int
                              Tile<BN>::SMEM_BYTES);
         done = true;
     }
-    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_tc_kernel<EPI, BN><<<grid, 128, Tile<BN>::SMEM_BYTES, st>>>(ma, mb, M, N, K, C, bias, ai, ao, vec);
+    // with column sums, a layer of blocks before the product's: two or more for each
+    // 128 columns of A, of which ceil(M / 64) have work
+    dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM);
+    if(g.colsum) {
+        grid.x = grid.x < 2 ? 2 : grid.x;
+        grid.z = 2;
+    }
+    gemm_tc_kernel<EPI, BN><<<grid, 128, Tile<BN>::SMEM_BYTES, st>>>(g.ma, g.mb, g.M, g.N, g.K, g.C, g.bias, g.aux_in,
+                                                                    g.aux_out, g.vec, g.a_mn, g.b_mn, g.colsum);
 }
 
-template<int BN>
-bool launch_epi(int epi, const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int K, void *C, const float *bias,
-                const __nv_bfloat16 *ai, __nv_bfloat16 *ao, int vec, cudaStream_t st)
+template<int BN> bool launch_epi(int epi, const GemmArgs &g, cudaStream_t st)
 {
     switch(epi) {
-    case BHCB_NN_EPI_F32: launch_gemm<BHCB_NN_EPI_F32, BN>(ma, mb, M, N, K, C, bias, ai, ao, vec, st); return true;
-    case BHCB_NN_EPI_BF16: launch_gemm<BHCB_NN_EPI_BF16, BN>(ma, mb, M, N, K, C, bias, ai, ao, vec, st); return true;
-    case BHCB_NN_EPI_BF16_GELU:
-        launch_gemm<BHCB_NN_EPI_BF16_GELU, BN>(ma, mb, M, N, K, C, bias, ai, ao, vec, st);
-        return true;
-    case BHCB_NN_EPI_BF16_DGELU:
-        launch_gemm<BHCB_NN_EPI_BF16_DGELU, BN>(ma, mb, M, N, K, C, bias, ai, ao, vec, st);
-        return true;
+    case BHCB_NN_EPI_F32: launch_gemm<BHCB_NN_EPI_F32, BN>(g, st); return true;
+    case BHCB_NN_EPI_BF16: launch_gemm<BHCB_NN_EPI_BF16, BN>(g, st); return true;
+    case BHCB_NN_EPI_BF16_GELU: launch_gemm<BHCB_NN_EPI_BF16_GELU, BN>(g, st); return true;
+    case BHCB_NN_EPI_BF16_DGELU: launch_gemm<BHCB_NN_EPI_BF16_DGELU, BN>(g, st); return true;
     default: return false;
     }
 }
@@ -436,29 +564,46 @@ bool launch_epi(int epi, const CUtensorMap &ma, const CUtensorMap &mb, int M, in
 
 using namespace bhcb;
 
-extern "C" int bhcb_nn_gemm(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t epi,
-                            const float *bias, const void *aux_in, void *aux_out, void *stream)
+extern "C" int bhcb_nn_gemm_t(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t a_t,
+                              int32_t b_t, int32_t epi, const float *bias, const void *aux_in, void *aux_out,
+                              float *colsum, void *stream)
 {
     if(!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return BHCB_ERR_ARG;
-    // TMA: 16-byte aligned bases and row strides (K a multiple of 8 bf16)
-    if((K % 8) != 0 || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    // TMA: 16-byte aligned bases and row strides (a multiple of 8 bf16)
+    if((K % 8) != 0 || (a_t && M % 8) || (b_t && N % 8) || (reinterpret_cast<uintptr_t>(A) & 15)
+       || (reinterpret_cast<uintptr_t>(B) & 15))
         return BHCB_ERR_ARG;
     if(epi == BHCB_NN_EPI_BF16_DGELU && !aux_in) return BHCB_ERR_ARG;
+    if(colsum && !a_t) return BHCB_ERR_ARG;
     // narrow tiles while one wave of them covers the output (148 SMs). At K = 1024,
     // wide and narrow: 128 tiles of 32 columns 19 and 13 us, 256 tiles 19 and 21 us
     const int bn = (long long)((M + BM - 1) / BM) * ((N + 31) / 32) <= 148 ? 32 : 128;
-    CUtensorMap ma, mb;
-    if(!make_map(&ma, A, M, K, BM) || !make_map(&mb, B, N, K, bn)) return BHCB_ERR_CUDA;
-    const __nv_bfloat16 *ai = reinterpret_cast<const __nv_bfloat16 *>(aux_in);
-    __nv_bfloat16 *ao = reinterpret_cast<__nv_bfloat16 *>(aux_out);
+    GemmArgs g{};
+    if(!(a_t ? make_map(&g.ma, A, K, M, BK, 64) : make_map(&g.ma, A, M, K, BM, BK))
+       || !(b_t ? make_map(&g.mb, B, K, N, BK, bn == 32 ? 32 : 64) : make_map(&g.mb, B, N, K, bn, BK)))
+        return BHCB_ERR_CUDA;
     const uintptr_t bases = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias)
         | reinterpret_cast<uintptr_t>(aux_in) | reinterpret_cast<uintptr_t>(aux_out);
-    const int vec = N % 8 == 0 && (bases & 15) == 0;
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.C = C;
+    g.bias = bias;
+    g.aux_in = reinterpret_cast<const __nv_bfloat16 *>(aux_in);
+    g.aux_out = reinterpret_cast<__nv_bfloat16 *>(aux_out);
+    g.vec = N % 8 == 0 && (bases & 15) == 0;
+    g.a_mn = a_t != 0;
+    g.b_mn = b_t != 0;
+    g.colsum = colsum;
     const cudaStream_t st = (cudaStream_t)stream;
-    if(!(bn == 32 ? launch_epi<32>(epi, ma, mb, M, N, K, C, bias, ai, ao, vec, st)
-                  : launch_epi<128>(epi, ma, mb, M, N, K, C, bias, ai, ao, vec, st)))
-        return BHCB_ERR_ARG;
+    if(!(bn == 32 ? launch_epi<32>(epi, g, st) : launch_epi<128>(epi, g, st))) return BHCB_ERR_ARG;
     return cudaGetLastError() == cudaSuccess ? BHCB_OK : BHCB_ERR_CUDA;
+}
+
+extern "C" int bhcb_nn_gemm(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t epi,
+                            const float *bias, const void *aux_in, void *aux_out, void *stream)
+{
+    return bhcb_nn_gemm_t(A, B, C, M, N, K, 0, 0, epi, bias, aux_in, aux_out, nullptr, stream);
 }
 
 extern "C" int bhcb_nn_status(int32_t *error, int32_t clear)

@@ -3,7 +3,6 @@
 // transpose, masked MSE loss and its gradient, bias gradients (column sums),
 // Adam updates of FP32 master weights with bf16 (and transposed bf16) copies,
 // FP32 -> bf16 conversion and the per-field RMS error used by the fallback.
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -11,8 +10,6 @@
 #include <cstdint>
 
 #include "../../include/bhcb.h"
-
-namespace cg = cooperative_groups;
 
 namespace bhcb {
 namespace {
@@ -101,58 +98,26 @@ __global__ void row_rms_kernel(const float *__restrict__ pred, const float *__re
     }
 }
 
-// db[n] = sum_m dy[m][n]. A warp sums every (32 x cluster)-th row of 64 columns
-// (one 128-byte line a row, 8 rows in flight), the warps' and then the cluster's
-// partial sums are added in order, through (distributed) shared memory: the
-// result does not depend on the schedule. One thread per column, which this
-// replaces, waited for memory row by row (32768 x 512: 1915 -> 18.5 us, 1.8 TB/s;
-// 256 x 1024: 18.5 -> 5 us).
-constexpr int CS_WARPS = 32, CS_COLS = 64, CS_CLUSTER = 8, CS_SPLIT_ROWS = 4096;
-template<bool VEC>
-__global__ void __launch_bounds__(CS_WARPS * 32) colsum_kernel(const __nv_bfloat16 *__restrict__ dy, int M, int N,
-                                                               float *__restrict__ db)
+// db[n] = sum_m dy[m][n], one row after another in FP32, 32 rows' loads in flight
+// per column. Waiting for each row by itself took 19 us for 256 x 32768, this 15.
+constexpr int CS_ROWS = 32;
+__global__ void __launch_bounds__(64) colsum_kernel(const __nv_bfloat16 *__restrict__ dy, int M, int N,
+                                                    float *__restrict__ db)
 {
-    __shared__ float part[CS_WARPS][CS_COLS];
-    __shared__ float sum[CS_COLS];
-    cg::cluster_group cl = cg::this_cluster();
-    const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-    const int n0 = (int)(blockIdx.x / (unsigned)nc) * CS_COLS + 2 * lane;
-    float s0 = 0.0f, s1 = 0.0f;
-    if(n0 < N) {
-        const bool two = n0 + 1 < N;
-        const __nv_bfloat16 *p = dy + n0;
-#pragma unroll 8
-        for(int m = rank * CS_WARPS + warp; m < M; m += nc * CS_WARPS) {
-            __nv_bfloat162 v;
-            if(VEC) {
-                v = *reinterpret_cast<const __nv_bfloat162 *>(p + (size_t)m * N);
-            } else {
-                v.x = p[(size_t)m * N];
-                v.y = two ? p[(size_t)m * N + 1] : __float2bfloat16_rn(0.0f);
-            }
-            s0 += __low2float(v);
-            s1 += __high2float(v);
-        }
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if(n >= N) return;
+    const __nv_bfloat16 *p = dy + n;
+    float s = 0.0f;
+    int m = 0;
+    for(; m + CS_ROWS <= M; m += CS_ROWS) {
+        __nv_bfloat16 v[CS_ROWS];
+#pragma unroll
+        for(int i = 0; i < CS_ROWS; ++i) v[i] = p[(size_t)(m + i) * N];
+#pragma unroll
+        for(int i = 0; i < CS_ROWS; ++i) s += __bfloat162float(v[i]);
     }
-    part[warp][2 * lane] = s0;
-    part[warp][2 * lane + 1] = s1;
-    __syncthreads();
-    const int col = (int)threadIdx.x;
-    if(col < CS_COLS) {
-        float s = 0.0f;
-#pragma unroll 8
-        for(int w = 0; w < CS_WARPS; ++w) s += part[w][col];
-        sum[col] = s;
-    }
-    cl.sync();
-    const int n = (int)(blockIdx.x / (unsigned)nc) * CS_COLS + col;
-    if(rank == 0 && col < CS_COLS && n < N) {
-        float s = 0.0f;
-        for(int r = 0; r < nc; ++r) s += *cl.map_shared_rank(&sum[col], r);
-        db[n] = s;
-    }
-    cl.sync();   // no block leaves while its sums are read
+    for(; m < M; ++m) s += __bfloat162float(p[(size_t)m * N]);
+    db[n] = s;
 }
 
 // Adam (bias-corrected) on FP32 master weights; writes the bf16 copy [R][C]
@@ -237,24 +202,8 @@ extern "C" int bhcb_nn_row_rms(const float *pred, const float *target, int32_t r
 extern "C" int bhcb_nn_colsum(const void *dy, int32_t M, int32_t N, float *db, void *stream)
 {
     if(!dy || !db || M <= 0 || N <= 0) return BHCB_ERR_ARG;
-    const int groups = (N + CS_COLS - 1) / CS_COLS;
-    // a cluster per 64 columns where a block's warps would take long turns at the rows
-    const int nc = M >= CS_SPLIT_ROWS ? CS_CLUSTER : 1;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = nc;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)groups * nc);
-    cfg.blockDim = dim3(CS_WARPS * 32);
-    cfg.stream = (cudaStream_t)stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    const bool vec = N % 2 == 0 && (reinterpret_cast<uintptr_t>(dy) & 3) == 0;
-    const __nv_bfloat16 *d = (const __nv_bfloat16 *)dy;
-    const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg, colsum_kernel<true>, d, M, N, db)
-                              : cudaLaunchKernelEx(&cfg, colsum_kernel<false>, d, M, N, db);
-    return e == cudaSuccess ? BHCB_OK : BHCB_ERR_CUDA;
+    colsum_kernel<<<(N + 63) / 64, 64, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)dy, M, N, db);
+    return NN_LAUNCH_OK;
 }
 
 extern "C" int bhcb_nn_adam(float *w, const float *g, float *m, float *v, int32_t rows, int32_t cols, float lr,

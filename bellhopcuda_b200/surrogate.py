@@ -108,12 +108,14 @@ class _Ops:
     def _p(t):
         return C.c_void_p(t.data_ptr()) if t is not None else None
 
-    def gemm(self, A, Bm, out, epi, bias=None, aux_in=None, aux_out=None):
-        M, K = A.shape
-        N = Bm.shape[0]
-        assert Bm.shape[1] == K and out.shape[0] == M and out.shape[1] == N
-        rc = self.lib.bhcb_nn_gemm(self._p(A), self._p(Bm), self._p(out), M, N, K, epi, self._p(bias),
-                                   self._p(aux_in), self._p(aux_out), self._s())
+    def gemm(self, A, Bm, out, epi, bias=None, aux_in=None, aux_out=None, a_t=False, b_t=False, colsum=None):
+        """out[M][N] = epilogue(A Bm^T); a_t, b_t: A is [K][M], Bm is [K][N] as stored;
+        colsum (with a_t): its sums over K."""
+        K, M = A.shape if a_t else A.shape[::-1]
+        N = Bm.shape[1 if b_t else 0]
+        assert Bm.shape[0 if b_t else 1] == K and out.shape[0] == M and out.shape[1] == N
+        rc = self.lib.bhcb_nn_gemm_t(self._p(A), self._p(Bm), self._p(out), M, N, K, a_t, b_t, epi, self._p(bias),
+                                     self._p(aux_in), self._p(aux_out), self._p(colsum), self._s())
         if rc != 0:
             raise BhcbError(rc, "bhcb_nn_gemm failed (M %d N %d K %d epi %d)" % (M, N, K, epi))
 
@@ -174,7 +176,7 @@ class _Ops:
 
 
 class Linear:
-    """y = act(x W^T + b): FP32 master weights with Adam states, bf16 W and W^T."""
+    """y = act(x W^T + b): FP32 master weights with Adam states, bf16 W."""
 
     def __init__(self, ops: _Ops, n_out: int, n_in: int, gelu: bool, rng: np.random.Generator, gain: float = 1.0):
         torch = ops.torch
@@ -189,12 +191,10 @@ class Linear:
         self.mw, self.vw = torch.zeros_like(self.w), torch.zeros_like(self.w)
         self.mb, self.vb = torch.zeros_like(self.b), torch.zeros_like(self.b)
         self.wb = torch.empty((n_out, n_in), dtype=torch.bfloat16, device=dev)
-        self.wt = torch.empty((n_in, n_out), dtype=torch.bfloat16, device=dev)
         self.refresh()
 
     def refresh(self):
         self.ops.to_bf16(self.w, self.wb)
-        self.ops.T(self.wb, self.wt)
 
     def params(self):
         return self.w.numel() + self.b.numel()
@@ -218,18 +218,19 @@ class Linear:
         Accumulates gw, gb; returns the gradient of pre_in (or None)."""
         torch = self.ops.torch
         M = x.shape[0]
-        dzt = self.ops.T(dz)                       # [n_out][M]
-        xt = self.ops.T(x)                         # [n_in][M]
-        self.ops.gemm(dzt, xt, self.gw, EPI_F32)   # gw = dz^T x
-        self.ops.colsum(dz, self.gb)
+        if self.n_out % 8 == 0:
+            self.ops.gemm(dz, x, self.gw, EPI_F32, a_t=True, b_t=True, colsum=self.gb)   # gw = dz^T x, gb = its sums
+        else:   # rows that TMA cannot step over: dz^T as a copy
+            self.ops.gemm(self.ops.T(dz), x, self.gw, EPI_F32, b_t=True)
+            self.ops.colsum(dz, self.gb)
         if pre_in is None:
             return None
         dpre = torch.empty((M, self.n_in), dtype=torch.bfloat16, device=x.device)
-        self.ops.gemm(dz, self.wt, dpre, EPI_DGELU, aux_in=pre_in)   # (dz W) * gelu'(pre_in)
+        self.ops.gemm(dz, self.wb, dpre, EPI_DGELU, aux_in=pre_in, b_t=True)   # (dz W) * gelu'(pre_in)
         return dpre
 
     def step(self, t: int, lr: float, wd: float = 0.0):
-        self.ops.adam(self.w, self.gw, self.mw, self.vw, t, lr, wb=self.wb, wt=self.wt, wd=wd)
+        self.ops.adam(self.w, self.gw, self.mw, self.vw, t, lr, wb=self.wb, wd=wd)
         self.ops.adam(self.b, self.gb, self.mb, self.vb, t, lr)
 
 
@@ -300,13 +301,10 @@ class Surrogate:
         torch = self.ops.torch
         B = dpred.shape[0]
         self.ops.colsum(dpred, self.gpb)
-        tbt = self.ops.T(self._tb)                      # [p][NP]
         db = torch.empty((B, self.p), dtype=torch.bfloat16, device="cuda")
-        self.ops.gemm(dpred, tbt, db, EPI_BF16)         # dL/db = dpred t
-        dpt = self.ops.T(dpred)                         # [NP][B]
-        bt = self.ops.T(self._b)                        # [p][B]
+        self.ops.gemm(dpred, self._tb, db, EPI_BF16, b_t=True)               # dL/db = dpred t
         dt = torch.empty((NP, self.p), dtype=torch.bfloat16, device="cuda")
-        self.ops.gemm(dpt, bt, dt, EPI_BF16)            # dL/dt = dpred^T b
+        self.ops.gemm(dpred, self._b, dt, EPI_BF16, a_t=True, b_t=True)      # dL/dt = dpred^T b
         self.branch.backward(db)
         self.trunk.backward(dt)
 

@@ -309,6 +309,11 @@ void bhcb_graph_destroy(bhcb_graph *graph);
 enum { BHCB_NN_EPI_F32 = 0, BHCB_NN_EPI_BF16 = 1, BHCB_NN_EPI_BF16_GELU = 2, BHCB_NN_EPI_BF16_DGELU = 3 };
 int bhcb_nn_gemm(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t epi,
                  const float *bias, const void *aux_in, void *aux_out, void *stream);
+/* The same product of operands stored transposed: A as [K,M] (a_t), B as [K,N]
+   (b_t); M, N then multiples of 8 as well. colsum (a_t only, may be NULL):
+   colsum[m] = sum over K of A[k][m] in FP32, in the order of k. */
+int bhcb_nn_gemm_t(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t a_t, int32_t b_t,
+                   int32_t epi, const float *bias, const void *aux_in, void *aux_out, float *colsum, void *stream);
 int bhcb_nn_status(int32_t *error, int32_t clear);
 /* Surrogate training / inference helpers (device pointers, enqueued on stream):
    tl_db: TL = -20 log10|p| of n complex64 pressures, clamped to [lo, hi];

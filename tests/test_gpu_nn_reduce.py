@@ -1,13 +1,13 @@
-"""The surrogate's reductions against float64: bias gradients (column sums of a
-bf16 matrix) and the squared-error loss with its gradient, at the edges of their
-splits (64 columns a block, 32 rows a turn, a cluster from 4096 rows on), for
-odd widths and unaligned bases.
+"""The surrogate's reductions: bias gradients (column sums of a bf16 matrix, which
+add one row after another in FP32 like numpy's accumulate) at the edges of their
+batches of 32 rows, and the squared-error loss with its gradient against float64,
+for odd sizes and unaligned bases.
 
-A column sum adds at most M / 32 + 40 terms one after another in FP32, each
-addition within 2^-24 of a partial sum that is at most sum |dy|. The loss is
-FP64: n * 2^-53 of it. The gradient is one bf16 rounding of scale * 2 d."""
+The loss is FP64: n * 2^-53 of it. The gradient is one bf16 rounding of
+scale * 2 d."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
 import bellhopcuda_b200 as B
@@ -24,7 +24,7 @@ def stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-@pytest.mark.parametrize("M", [1, 31, 33, 256, 4095, 4096, 32768])
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 256, 4100])
 @pytest.mark.parametrize("N,shift", [(1, 0), (8, 0), (63, 0), (64, 1), (66, 0), (512, 0)])
 def test_colsum(M, N, shift):
     import torch
@@ -32,9 +32,8 @@ def test_colsum(M, N, shift):
     dy = torch.randn(M * N + shift, device="cuda", generator=g).bfloat16()[shift:].view(M, N)
     db = torch.full((N + 1,), 7.0, device="cuda")
     assert B.load_library().bhcb_nn_colsum(ptr(dy), M, N, ptr(db), stream()) == 0
-    d = dy.double()
-    bound = (M / 32 + 40) * 2.0 ** -24 * d.abs().sum(0)
-    assert bool(((db[:N].double() - d.sum(0)).abs() <= bound).all()) and db[N].item() == 7.0
+    ref = np.add.accumulate(dy.float().cpu().numpy(), axis=0)[-1]
+    assert np.array_equal(db[:N].cpu().numpy(), ref) and db[N].item() == 7.0
 
 
 @pytest.mark.parametrize("n,shift", [(1, 0), (3, 0), (255, 1), (1024, 0), (1027, 0), (2097155, 0), (300000, 1)])
