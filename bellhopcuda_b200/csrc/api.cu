@@ -19,6 +19,7 @@
 #include "host/env2d.h"
 #include "host/rt.h"
 #include "host/run3d.h"
+#include "hostcopy.h"
 #include "noalloc.h"
 #include "tabstage.cuh"
 
@@ -133,6 +134,7 @@ struct bhcb_ctx {
     uint64_t max_memory = 16ull << 30;
     void (*output_cb)(const char *) = nullptr;
     cudaStream_t stream = nullptr;
+    HostCopy host;                    // large results on their way to pageable memory
     cudaStream_t stream2 = nullptr;   // influence launches beside the trace
     bool overlap = false;             // mixed TL runs: influence overlaps the trace (BHCB_FLAG_OVERLAP_INFLUENCE)
     // pipelined TL steps (BHCB_FLAG_PIPELINE): slot k % 2 of launch k; slot 0
@@ -1026,7 +1028,7 @@ void trace_rays(bhcb_ctx *c, RaySet &R)
         }
         R.rz.resize(2 * (size_t)tot);
         if(tot)
-            CK(cudaMemcpyAsync(R.rz.data(), pts_d.p, tot * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+            CK(c->host.copy(R.rz.data(), pts_d.p, tot * sizeof(double2), c->stream));
         CK(cudaStreamSynchronize(c->stream));
         if(once) {
             long long to = 0;
@@ -1726,7 +1728,7 @@ int bhcb_copy_field(bhcb_ctx *c, int32_t env, int32_t ifreq, void *dst, size_t b
         const Field *F = find_field(c, env, ifreq);
         size_t need = (size_t)F->nsz * F->nrzp * F->nrr * sizeof(float2);
         if(!dst || bytes < need) throw std::invalid_argument("destination too small");
-        CK(cudaMemcpyAsync(dst, (float2 *)c->out.p + F->base, need, cudaMemcpyDeviceToHost, c->stream));
+        CK(c->host.copy(dst, (float2 *)c->out.p + F->base, need, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         return BHCB_OK;
     });
@@ -1817,8 +1819,7 @@ int bhcb_copy_arrivals(bhcb_ctx *c, int32_t env, int32_t ifreq, int32_t *narr, s
         if(arr) {
             size_t need = cells * (size_t)c->max_narr * sizeof(ArrivalRec);
             if(arr_bytes < need) throw std::invalid_argument("arrival buffer too small");
-            CK(cudaMemcpyAsync(arr, (ArrivalRec *)c->arr_d.p + (size_t)F->base * c->max_narr, need,
-                               cudaMemcpyDeviceToHost, c->stream));
+            CK(c->host.copy(arr, (ArrivalRec *)c->arr_d.p + (size_t)F->base * c->max_narr, need, c->stream));
         }
         CK(cudaStreamSynchronize(c->stream));
         return BHCB_OK;

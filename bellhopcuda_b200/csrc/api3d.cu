@@ -16,6 +16,7 @@
 #include "host/env2d.h"
 #include "host/rt.h"
 #include "host/run3d.h"
+#include "hostcopy.h"
 
 namespace bhcb {
 
@@ -80,6 +81,7 @@ struct Run3 {
     std::vector<Env3Slot> envs;
     std::vector<GroupDev> groups_h;
     DevBuf arena, groups_d, segs, counters, field;
+    HostCopy host;                    // large results on their way to pageable memory
     long long njobs = 0;
     unsigned long long seg_cap = 0;
     int64_t total_field = 0;   // receiver cells of the batch
@@ -666,7 +668,7 @@ uint32_t trace_rays3(Run3 *r, RaySet3 &R, cudaStream_t st, uint32_t &warn_bits)
     CK(rays(G, ng, (const long long *)jobs_d.p, (const int *)lim_d.p, n, (const long long *)off_d.p,
                      (double *)pts_d.p, (int *)npts_d.p, (int *)bnc_d.p, ctr, false, r->sm_count, st));
     R.xyz.resize(3 * (size_t)tot);
-    if(tot) CK(cudaMemcpyAsync(R.xyz.data(), pts_d.p, tot * 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if(tot) CK(r->host.copy(R.xyz.data(), pts_d.p, tot * 3 * sizeof(double), st));
     CK(cudaStreamSynchronize(st));
     return 0;
 }
@@ -766,7 +768,7 @@ void run3_copy_field(Run3 *r, int env, void *dst, size_t bytes, cudaStream_t st)
         throw StateError("not a TL run: use bhcb_copy_arrivals / bhcb_eigen_hits / bhcb_copy_rays");
     const size_t need = (size_t)S.field_n * sizeof(float2);
     if(!dst || bytes < need) throw std::invalid_argument("destination too small");
-    CK(cudaMemcpyAsync(dst, (float2 *)r->field.p + S.field_base, need, cudaMemcpyDeviceToHost, st));
+    CK(r->host.copy(dst, (float2 *)r->field.p + S.field_base, need, st));
     CK(cudaStreamSynchronize(st));
 }
 
@@ -823,8 +825,7 @@ void run3_copy_arrivals(Run3 *r, int env, int32_t *narr, size_t narr_bytes, void
     if(arr) {
         const size_t need = cells * (size_t)r->max_narr * sizeof(ArrivalRec);
         if(arr_bytes < need) throw std::invalid_argument("arrival buffer too small");
-        CK(cudaMemcpyAsync(arr, (ArrivalRec *)r->arr_d.p + (size_t)S.field_base * r->max_narr, need,
-                           cudaMemcpyDeviceToHost, st));
+        CK(r->host.copy(arr, (ArrivalRec *)r->arr_d.p + (size_t)S.field_base * r->max_narr, need, st));
     }
     CK(cudaStreamSynchronize(st));
 }
