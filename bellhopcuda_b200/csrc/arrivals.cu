@@ -15,8 +15,8 @@
 //      with a 64-bit key (receiver cell, ray, step) for arrivals or (field,
 //      ray, step, column walk position, depth) for eigen hits;
 //   3. a stable LSD radix sort of the keys (8-bit digits; per-tile histograms,
-//      one exclusive scan, warp-stable scatter);
-//   4. arr_replay_kernel: one thread per receiver cell applies the AddArr rule
+//      an exclusive scan per digit, warp-stable scatter);
+//   4. arr_replay_kernel: one warp per receiver cell applies the AddArr rule
 //      to its candidates in sorted order, then PostProcessArrivals' amplitude
 //      scaling (src/mode/arr.cpp:24-74); eigen_emit_kernel writes the hits in
 //      sorted order.
@@ -37,7 +37,7 @@ namespace bhcb {
 namespace {
 
 constexpr double RAD_DEG = 180.0 / BHCB_PI;
-constexpr int SORT_TILE = 4096;   // keys per scatter tile (one warp)
+constexpr int SORT_TILE = 1024;   // keys per scatter tile (one warp)
 
 __device__ __forceinline__ int group_of_cell(const GroupDev *groups, int ngroups, long long cell)
 {
@@ -176,29 +176,43 @@ __global__ void rs_hist_kernel(const uint64_t *__restrict__ keys, unsigned long 
     for(int d = threadIdx.x; d < 256; d += blockDim.x) hist[(size_t)d * ntiles + tile] = h[d];
 }
 
-// exclusive scan of len entries in one block of 1024 threads
-__global__ void __launch_bounds__(1024) rs_scan_kernel(uint32_t *a, long long len)
+// One block per digit: exclusive scan of its ntiles counts; its total goes to
+// hist[256 ntiles + digit], and the scatter adds the digits before it. One block
+// of 1024 threads over all digits took 650 us for 1553 tiles, this 6.
+__global__ void __launch_bounds__(256) rs_scan_kernel(uint32_t *hist, int ntiles)
 {
-    __shared__ uint32_t part[1024];
-    __shared__ uint32_t carry;
-    if(threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for(long long base = 0; base < len; base += 1024) {
-        const long long i = base + threadIdx.x;
-        const uint32_t v = i < len ? a[i] : 0u;
-        part[threadIdx.x] = v;
-        __syncthreads();
-        for(int off = 1; off < 1024; off <<= 1) {   // Hillis-Steele inclusive scan
-            uint32_t t = threadIdx.x >= off ? part[threadIdx.x - off] : 0u;
-            __syncthreads();
-            part[threadIdx.x] += t;
-            __syncthreads();
+    __shared__ uint32_t part[8];
+    uint32_t *a = hist + (size_t)blockIdx.x * ntiles;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for(int base = 0; base < ntiles; base += 1024) {
+        const int i = base + 4 * (int)threadIdx.x;
+        uint32_t v[4], sum = 0;
+        for(int j = 0; j < 4; ++j) {
+            v[j] = i + j < ntiles ? a[i + j] : 0u;
+            sum += v[j];
         }
-        if(i < len) a[i] = carry + part[threadIdx.x] - v;
+        uint32_t x = sum;
+        for(int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= o) x += t;
+        }
+        if(lane == 31) part[w] = x;
         __syncthreads();
-        if(threadIdx.x == 1023) carry += part[1023];
+        uint32_t before = carry, all = 0;
+        for(int j = 0; j < 8; ++j) {
+            if(j < w) before += part[j];
+            all += part[j];
+        }
+        before += x - sum;
+        for(int j = 0; j < 4; ++j) {
+            if(i + j < ntiles) a[i + j] = before;
+            before += v[j];
+        }
+        carry += all;
         __syncthreads();
     }
+    if(threadIdx.x == 0) hist[(size_t)256 * ntiles + blockIdx.x] = carry;
 }
 
 // stable scatter: one warp per tile, 32 keys at a time in order; lanes with the
@@ -210,7 +224,21 @@ __global__ void __launch_bounds__(32) rs_scatter_kernel(
 {
     __shared__ uint32_t off[256];
     const int tile = blockIdx.x, lane = threadIdx.x;
-    for(int d = lane; d < 256; d += 32) off[d] = hist[(size_t)d * ntiles + tile];
+    {   // lane: digits 8 lane ... + 7
+        const uint32_t *total = hist + (size_t)256 * ntiles + 8 * lane;
+        uint32_t sum = 0, x;
+        for(int j = 0; j < 8; ++j) sum += total[j];
+        x = sum;
+        for(int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= o) x += t;
+        }
+        x -= sum;
+        for(int j = 0; j < 8; ++j) {
+            off[8 * lane + j] = x + hist[(size_t)(8 * lane + j) * ntiles + tile];
+            x += total[j];
+        }
+    }
     __syncwarp();
     const unsigned long long b = (unsigned long long)tile * SORT_TILE;
     const unsigned long long e = min(n, b + SORT_TILE);
@@ -246,114 +274,145 @@ __global__ void __launch_bounds__(32) rs_scatter_kernel(
 // D3: 3-D run (source angles from the 3-D job, receiver azimuth from the
 // candidate, no amplitude scaling); the replay continues from the counts
 // already in narr_out, so job-ordered waves compose.
+// One warp per cell: 32 candidates are loaded at once, and applied in order from
+// there by all lanes together, the owner of each writing. The last arrival, which
+// the next may merge with, stays in registers; the weakest of a full cell is
+// found by all lanes and kept until an arrival changes. One thread per cell
+// waited for memory at every candidate and at each of the max_narr amplitudes:
+// 614k candidates of 4141 cells 1946 us, so 319; 6.36 M of 45000 (3-D) 2702 and 1138.
 template<bool D3>
-__global__ void arr_replay_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals,
-                                  const ArrCand *__restrict__ cands, unsigned long long n,
-                                  const GroupDev *__restrict__ groups, int ngroups,
-                                  const double *__restrict__ freqs, long long ncells, int sh_cell,
-                                  int max_narr, int allow_merging, int32_t *narr_out, ArrivalRec *arr_out)
+__global__ void __launch_bounds__(128) arr_replay_kernel(
+    const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, const ArrCand *__restrict__ cands,
+    unsigned long long n, const GroupDev *__restrict__ groups, int ngroups, const double *__restrict__ freqs,
+    long long ncells, int sh_cell, int max_narr, int allow_merging, int32_t *narr_out, ArrivalRec *arr_out)
 {
-    for(long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < ncells;
-        cell += (long long)gridDim.x * blockDim.x) {
-        // candidate range of this cell in the sorted keys
-        const uint64_t klo = (uint64_t)cell << sh_cell, khi = (uint64_t)(cell + 1) << sh_cell;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = (int)(threadIdx.x & 31);
+    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    for(long long cell = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); cell < ncells;
+        cell += nwarps) {
+        // candidate range of this cell in the sorted keys: even lanes its begin, odd its end
+        const uint64_t want = (uint64_t)(cell + (lane & 1)) << sh_cell;
         unsigned long long lo = 0, hi = n;
         while(lo < hi) {
             unsigned long long m = (lo + hi) >> 1;
-            if(keys[m] < klo) lo = m + 1; else hi = m;
+            if(keys[m] < want) lo = m + 1; else hi = m;
         }
-        const unsigned long long begin = lo;
-        hi = n;
-        while(lo < hi) {
-            unsigned long long m = (lo + hi) >> 1;
-            if(keys[m] < khi) lo = m + 1; else hi = m;
-        }
-        const unsigned long long end = lo;
+        const unsigned long long begin = __shfl_sync(ALL, lo, 0), end = __shfl_sync(ALL, lo, 1);
         const GroupDev &G = groups[group_of_cell(groups, ngroups, cell)];
         const double omega = D3 ? 2.0 * BHCB_PI * G.env3->freq0 : 2.0 * BHCB_PI * freqs[G.freq_base];
         ArrivalRec *ba = arr_out + (size_t)cell * max_narr;
         int nt = D3 ? narr_out[cell] : 0;
-        for(unsigned long long k = begin; k < end; ++k) {
-            const ArrCand &c = cands[vals[k]];
-            double src_decl, src_azim_d = 0.0;
-            float rcvr_azim;
-            if(D3) {
-                const Job3 J = job_indices3(*G.env3, (int)((long long)c.job - G.job_base));
-                src_decl = RAD_DEG * G.env3->alpha[J.ialpha];
-                src_azim_d = RAD_DEG * G.env3->beta[J.ibeta];
-                rcvr_azim = c.rcvr_azim;
-            } else {
-                src_decl = RAD_DEG * G.env->alpha[c.aux];
-                rcvr_azim = __int_as_float(0x7fc00000);   // NaN: no azimuth in 2-D
-            }
-            const float azim = D3 ? (float)src_azim_d : __int_as_float(0x7fc00000);
-            if(allow_merging) {
-                const float PhaseTol = 0.05f;
-                bool second = false;
-                if(nt >= 1) {
-                    const ArrivalRec &L = ba[nt - 1];
-                    const double ddr = c.delay_re - (double)L.delay_re, ddi = c.delay_im - (double)L.delay_im;
-                    second = omega * hypot(ddr, ddi) < (double)PhaseTol
-                             && fabs((double)L.Phase - c.phase) < (double)PhaseTol;
-                }
-                if(!second) {
-                    int iArr;
-                    if(nt >= max_narr) {
-                        iArr = -1;
-                        double weakest = c.amp;
-                        for(int j = 0; j < max_narr; ++j)
-                            if((double)ba[j].a < weakest) {
-                                weakest = (double)ba[j].a;
-                                iArr = j;
-                            }
-                        if(iArr < 0) continue;
-                    } else {
-                        iArr = nt++;
-                    }
-                    ArrivalRec &A = ba[iArr];
-                    A.a = (float)c.amp;
-                    A.Phase = (float)c.phase;
-                    A.delay_re = (float)c.delay_re;
-                    A.delay_im = (float)c.delay_im;
-                    A.SrcDeclAngle = (float)src_decl;
-                    A.SrcAzimAngle = azim;
-                    A.RcvrDeclAngle = c.rcvr_decl;
-                    A.RcvrAzimAngle = rcvr_azim;
-                    A.NTopBnc = c.ntop;
-                    A.NBotBnc = c.nbot;
+        // of the last arrival
+        float l_re = 0.f, l_im = 0.f, l_ph = 0.f;
+        if(nt >= 1) {
+            const ArrivalRec &L = ba[min(nt, max_narr) - 1];
+            l_re = L.delay_re;
+            l_im = L.delay_im;
+            l_ph = L.Phase;
+        }
+        int weak_j = -1;         // weakest arrival of a full cell; -1: to be found
+        float weak = 0.f;
+        for(unsigned long long k0 = begin; k0 < end; k0 += 32) {
+            const int cnt = (int)min((unsigned long long)32, end - k0);
+            ArrCand c{};
+            ArrivalRec A;
+            if(lane < cnt) {
+                c = cands[vals[k0 + lane]];
+                double src_decl;
+                if(D3) {
+                    const Job3 J = job_indices3(*G.env3, (int)((long long)c.job - G.job_base));
+                    src_decl = RAD_DEG * G.env3->alpha[J.ialpha];
+                    A.SrcAzimAngle = (float)(RAD_DEG * G.env3->beta[J.ibeta]);
+                    A.RcvrAzimAngle = c.rcvr_azim;
                 } else {
-                    ArrivalRec &A = ba[nt - 1];
-                    const float amp = (float)c.amp;
-                    const float tot = __fadd_rn(A.a, amp);
-                    const float w1 = __fdiv_rn(A.a, tot), w2 = __fdiv_rn(amp, tot);
-                    A.delay_re = __fadd_rn(__fmul_rn(w1, A.delay_re), __fmul_rn(w2, (float)c.delay_re));
-                    A.delay_im = __fadd_rn(__fmul_rn(w1, A.delay_im), __fmul_rn(w2, (float)c.delay_im));
-                    A.a = tot;
-                    A.SrcDeclAngle = __fadd_rn(__fmul_rn(w1, A.SrcDeclAngle), __fmul_rn(w2, (float)src_decl));
-                    A.SrcAzimAngle = __fadd_rn(__fmul_rn(w1, A.SrcAzimAngle), __fmul_rn(w2, azim));
-                    A.RcvrDeclAngle = __fadd_rn(__fmul_rn(w1, A.RcvrDeclAngle), __fmul_rn(w2, c.rcvr_decl));
-                    A.RcvrAzimAngle = __fadd_rn(__fmul_rn(w1, A.RcvrAzimAngle), __fmul_rn(w2, rcvr_azim));
+                    src_decl = RAD_DEG * G.env->alpha[c.aux];
+                    A.SrcAzimAngle = A.RcvrAzimAngle = __int_as_float(0x7fc00000);   // NaN: no azimuth in 2-D
                 }
-            } else {
-                const int j = nt++;
-                if(j >= max_narr) continue;
-                ArrivalRec &A = ba[j];
                 A.a = (float)c.amp;
                 A.Phase = (float)c.phase;
                 A.delay_re = (float)c.delay_re;
                 A.delay_im = (float)c.delay_im;
                 A.SrcDeclAngle = (float)src_decl;
-                A.SrcAzimAngle = azim;
                 A.RcvrDeclAngle = c.rcvr_decl;
-                A.RcvrAzimAngle = rcvr_azim;
                 A.NTopBnc = c.ntop;
                 A.NBotBnc = c.nbot;
             }
+            if(!allow_merging) {
+                if(lane < cnt && nt + lane < max_narr) ba[nt + lane] = A;
+                nt = min(nt + cnt, max_narr);
+                continue;
+            }
+            for(int i = 0; i < cnt; ++i) {
+                const double phase = __shfl_sync(ALL, c.phase, i), dre = __shfl_sync(ALL, c.delay_re, i);
+                const double dim = __shfl_sync(ALL, c.delay_im, i);
+                bool second = false;
+                const float PhaseTol = 0.05f;
+                if(nt >= 1 && fabs((double)l_ph - phase) < (double)PhaseTol) {
+                    const double ddr = dre - (double)l_re, ddi = dim - (double)l_im;
+                    // hypot is at least the larger part, within its rounding
+                    second = omega * fabs(ddr) < 1.0 && omega * hypot(ddr, ddi) < (double)PhaseTol;
+                }
+                if(!second) {
+                    int slot = nt;
+                    if(nt >= max_narr) {
+                        if(weak_j < 0) {
+                            __syncwarp();
+                            weak = __int_as_float(0x7f800000);
+                            weak_j = 0x7fffffff;
+                            for(int j = lane; j < max_narr; j += 32)
+                                if(ba[j].a < weak) {
+                                    weak = ba[j].a;
+                                    weak_j = j;
+                                }
+                            for(int o = 16; o > 0; o >>= 1) {
+                                const float v = __shfl_xor_sync(ALL, weak, o);
+                                const int j = __shfl_xor_sync(ALL, weak_j, o);
+                                if(v < weak || (v == weak && j < weak_j)) {
+                                    weak = v;
+                                    weak_j = j;
+                                }
+                            }
+                        }
+                        if(!((double)weak < __shfl_sync(ALL, c.amp, i))) continue;
+                        slot = weak_j;
+                        weak_j = -1;
+                    } else {
+                        ++nt;
+                    }
+                    if(lane == i) ba[slot] = A;
+                    if(slot == nt - 1) {
+                        l_re = (float)dre;
+                        l_im = (float)dim;
+                        l_ph = (float)phase;
+                    }
+                } else {
+                    __syncwarp();
+                    if(lane == i) {
+                        ArrivalRec &L = ba[nt - 1];
+                        const float tot = __fadd_rn(L.a, A.a);
+                        const float w1 = __fdiv_rn(L.a, tot), w2 = __fdiv_rn(A.a, tot);
+                        l_re = __fadd_rn(__fmul_rn(w1, L.delay_re), __fmul_rn(w2, A.delay_re));
+                        l_im = __fadd_rn(__fmul_rn(w1, L.delay_im), __fmul_rn(w2, A.delay_im));
+                        L.delay_re = l_re;
+                        L.delay_im = l_im;
+                        L.a = tot;
+                        L.SrcDeclAngle = __fadd_rn(__fmul_rn(w1, L.SrcDeclAngle), __fmul_rn(w2, A.SrcDeclAngle));
+                        L.SrcAzimAngle = __fadd_rn(__fmul_rn(w1, L.SrcAzimAngle), __fmul_rn(w2, A.SrcAzimAngle));
+                        L.RcvrDeclAngle = __fadd_rn(__fmul_rn(w1, L.RcvrDeclAngle), __fmul_rn(w2, A.RcvrDeclAngle));
+                        L.RcvrAzimAngle = __fadd_rn(__fmul_rn(w1, L.RcvrAzimAngle), __fmul_rn(w2, A.RcvrAzimAngle));
+                    }
+                    l_re = __shfl_sync(ALL, l_re, i);
+                    l_im = __shfl_sync(ALL, l_im, i);
+                    weak_j = -1;
+                }
+            }
         }
+        __syncwarp();
         // PostProcessArrivals (src/mode/arr.cpp:24-74): clamp the count; 2-D
         // and Nx2D scale the amplitudes (3-D factor 1)
         if(nt > max_narr) nt = max_narr;
-        narr_out[cell] = nt;
+        if(lane == 0) narr_out[cell] = nt;
         if(D3 && !G.env3->nx2d) continue;
         // 2-D rays (2-D and Nx2D): cylindrical spreading per receiver range,
         // the last index of both field layouts
@@ -364,7 +423,7 @@ __global__ void arr_replay_kernel(const uint64_t *__restrict__ keys, const uint3
         if(!D3 && G.env->line_source) factor = (float)(FLTD(4.0) * sqrt(BHCB_PI));
         else if(fabs(rr[ir]) < DBL_EPS) factor = 1e5f;
         else factor = (float)(FLTD(1.0) / sqrt(rr[ir]));
-        for(int j = 0; j < nt; ++j) ba[j].a = __fmul_rn(ba[j].a, factor);
+        for(int j = lane; j < nt; j += 32) ba[j].a = __fmul_rn(ba[j].a, factor);
     }
 }
 
@@ -426,7 +485,7 @@ template cudaError_t launch_arr_gather<double>(const void *, unsigned long long,
 
 size_t radix_sort_hist_entries(unsigned long long n)
 {
-    return (size_t)256 * (size_t)((n + SORT_TILE - 1) / SORT_TILE);
+    return (size_t)256 * (size_t)((n + SORT_TILE - 1) / SORT_TILE) + 256;
 }
 
 // Sorts (keys, vals) by the low `bits` bits of the keys; the result is in
@@ -442,7 +501,7 @@ cudaError_t radix_sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t 
     int passes = 0;
     for(int shift = 0; shift < bits; shift += 8, ++passes) {
         rs_hist_kernel<<<ntiles, 256, 0, st>>>(ki, n, shift, hist, ntiles);
-        rs_scan_kernel<<<1, 1024, 0, st>>>(hist, (long long)256 * ntiles);
+        rs_scan_kernel<<<256, 256, 0, st>>>(hist, ntiles);
         rs_scatter_kernel<<<ntiles, 32, 0, st>>>(ki, vi, ko, vo, n, shift, hist, ntiles);
         std::swap(ki, ko);
         std::swap(vi, vo);
@@ -456,7 +515,7 @@ cudaError_t launch_arr_replay(const uint64_t *keys, const uint32_t *vals, const 
                               int max_narr, int allow_merging, int32_t *narr, ArrivalRec *arr, int sm_count,
                               cudaStream_t st, bool d3)
 {
-    long long grid = (ncells + 127) / 128;
+    long long grid = (ncells + 3) / 4;
     if(grid > (long long)sm_count * 64) grid = (long long)sm_count * 64;
     if(grid < 1) grid = 1;
     if(d3)
