@@ -959,9 +959,10 @@ int group_of_field(const bhcb_ctx *c, int fi)
 }
 
 // Trajectories of R.jobs (limits as for the ray kernel). A ray with a limit has
-// at most limit + 3 points, so eigenrays are traced once, into as much room (a pass of two saved), and
-// packed as they leave; rays without one are counted by a pass of their own,
-// which sizes the buffer of a second pass of the same deterministic trace.
+// at most limit + 3 points, so eigenrays are traced once, into as much room (one
+// pass of two saved), and packed as they leave; rays without one are counted by a
+// pass of their own, which sizes the buffer of a second pass of the same
+// deterministic trace.
 void trace_rays(bhcb_ctx *c, RaySet &R)
 {
     const int n = (int)R.jobs.size();

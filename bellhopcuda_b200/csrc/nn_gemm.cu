@@ -181,7 +181,7 @@ __device__ __forceinline__ uint4 pack_bf16(const float *x)
 // rows one after another in FP32, as one thread per column would add them (the
 // weights' later roundings hang on the last bits of these sums). TMA fills the
 // ring; two warps add 32 columns each, sixteen rows read ahead of the additions,
-// 7 cycles a row in all: 32768 rows in 120 us beside a product of 75
+// 7 cycles a row in all: 32768 rows in 120 us beside a product of 82
 // (a column per thread from global memory took 1915).
 template<int BN>
 __device__ __forceinline__ void column_sums(uint8_t *ring, uint64_t *full, uint64_t *empty, const CUtensorMap *tmA,
