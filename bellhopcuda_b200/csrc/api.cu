@@ -396,6 +396,16 @@ bool all_seg(const bhcb_ctx *c, int g0, int g1)
     return true;
 }
 
+// The receiver ranges are rr[0] + i delta_r, as the ray-centred beams' index of a
+// range (RToIR) takes them to be. delta_r is the last spacing, so a list of ranges
+// need not agree with it.
+bool even_ranges(const EnvTables &T)
+{
+    for(size_t i = 0; i < T.rr.size(); ++i)
+        if(!(std::fabs(T.rr[i] - (T.rr[0] + (double)i * T.delta_r)) <= 5e-7 * T.delta_r)) return false;
+    return true;
+}
+
 // Packed segments of a profile of type C, S or P; empty for other types, for
 // complex sound speeds and for fewer than two nodes.
 std::vector<SspSeg> pack_segments(const EnvTables &T)
@@ -541,6 +551,7 @@ void do_prepare(bhcb_ctx *c)
         d.isingle = T.isingle;
         d.dalpha = T.dalpha;
         d.delta_r = T.delta_r;
+        d.rr_even = even_ranges(T);
         d.deltas = T.deltas;
         d.box_x = T.box_x;
         d.box_y = T.box_y;

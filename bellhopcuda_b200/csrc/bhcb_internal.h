@@ -61,7 +61,8 @@ struct EnvDev {
     const double *c, *cz;      // complex, interleaved re/im, [nssp]
     const double *n2, *n2z;    // complex [nssp]
     const double *coef;        // complex [4][nssp]: spline (S) or pchip (P) coefficients
-    int32_t has_seg, pad_s;    // segtab holds the profile: type C, S or P, no attenuation
+    int32_t has_seg;           // segtab holds the profile: type C, S or P, no attenuation
+    int32_t rr_even;           // every rr[i] is rr[0] + i delta_r, to 5e-7 of delta_r
     const SspSeg *segtab;      // [nssp - 1]
     // quad (range-dependent) SSP (src/ssp.hpp:157-212): profile ranges qr[nqr]
     // (m), sound speed qc[iz * nqr + ir] and its depth gradient qcz[iz * nqr + ir]

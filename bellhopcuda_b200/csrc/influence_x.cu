@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(32 * RCW) influence_raycen_kernel(
             r.fl = gauss ? min(FLTD(0.2) * freq * S.tau1r, BHCB_PI * (S.c0 / freq)) : 0.0;
             // over s in [-0.002, 1.002], rounding included
             const double q = max(fabs(r.q0), fabs(r.q0 + r.dq)) + 0.002 * fabs(r.dq);
-            r.reach = 1.000001 * W * max(fabs(q * r.rcp), r.fl);
+            r.reach = e.rr_even ? 1.000001 * W * max(fabs(q * r.rcp), r.fl) : (double)INFINITY;
             r.amp = S.amp; r.ph_a = S.ph_a; r.ph_b = S.ph_b;
             r.t0r = S.tau0r; r.t0i = S.tau0i; r.dtr = S.dtaur; r.dti = S.dtaui;
             const double px = __shfl_up_sync(0xffffffffu, r.xb, 1), pz = __shfl_up_sync(0xffffffffu, r.zb, 1);
@@ -644,8 +644,9 @@ __global__ void __launch_bounds__(32 * RCW) influence_raycen_kernel(
                 ir = irA + up;
                 end = irB + up;
                 dir = 2 * up - 1;
-                // the whole record out of reach: no receiver lies beyond its ends by more
-                // than 1e-6 of the spacing (rtoir), 0.001 of the distance in r here
+                // the whole record out of reach: no receiver of an even grid lies beyond its
+                // ends by more than 1e-6 of the spacing (rtoir) and 5e-7 (rr_even), 0.0015 of
+                // the distance in r here; on an uneven one the two ends bound nothing
                 const double dn = nB - nA;
                 if(fabs(rB - rA) > 1e-3 * delta && (nA > 0.0) == (nB > 0.0)
                    && min(fabs(nA), fabs(nB)) - 0.002 * fabs(dn) > S.reach)
