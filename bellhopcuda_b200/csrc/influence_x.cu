@@ -571,7 +571,10 @@ __global__ void __launch_bounds__(32 * RCW) influence_raycen_kernel(
             r.fl = gauss ? min(FLTD(0.2) * freq * S.tau1r, BHCB_PI * (S.c0 / freq)) : 0.0;
             // over s in [-0.002, 1.002], rounding included
             const double q = max(fabs(r.q0), fabs(r.q0 + r.dq)) + 0.002 * fabs(r.dq);
-            r.reach = e.rr_even ? 1.000001 * W * max(fabs(q * r.rcp), r.fl) : (double)INFINITY;
+            // a beam that is not a number (a hat; a Gaussian falls back to its least sigma)
+            // reaches every receiver, as in the test per receiver
+            const double sq = fabs(q * r.rcp);
+            r.reach = e.rr_even && (gauss || sq == sq) ? 1.000001 * W * max(sq, r.fl) : (double)INFINITY;
             r.amp = S.amp; r.ph_a = S.ph_a; r.ph_b = S.ph_b;
             r.t0r = S.tau0r; r.t0i = S.tau0i; r.dtr = S.dtaur; r.dti = S.dtaui;
             const double px = __shfl_up_sync(0xffffffffu, r.xb, 1), pz = __shfl_up_sync(0xffffffffu, r.zb, 1);
