@@ -148,9 +148,10 @@ template<typename R, typename RecR> __device__ __forceinline__ bool infl_prologu
     const RayPt<R> &pp = e.gaussian ? p1 : p0;
     rec.phase_a = (RecR)((double)pp.Phase + inf.phase);
     rec.phase_b = (RecR)(inf.phase + BHCB_PI / FLTD(2.0));
-    // max|q| rcp_q0 / |tx|; a vertical segment (tx 0 or negligible) keeps IEEE division's infinity
+    // max|q| rcp_q0 / |tx|; a vertical segment (tx 0 or negligible) and a spreading that has grown
+    // past any range (rays caught on a concave bottom: infinite in the end) keep IEEE division's infinity
     const R qmax = max(fabs(p0.q.x), fabs(p1.q.x)) * rcp_q0;
-    if(sizeof(R) == 8 && atx > 1.0e-100) rec.sigma_seg = (RecR)div_rn((double)qmax, atx);
+    if(sizeof(R) == 8 && atx > 1.0e-100 && (double)qmax < 1.0e200) rec.sigma_seg = (RecR)div_rn((double)qmax, atx);
     else rec.sigma_seg = (RecR)(qmax / (R)atx);
     rec.c0 = (RecR)p0.c;
     rec.tau1r = (RecR)p1.taur;

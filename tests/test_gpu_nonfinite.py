@@ -1,8 +1,8 @@
 """Beams whose spreading is not a finite number: a receiver test that compares with
 NaN or infinity keeps the receiver, and so must every rule that leaves out work.
 
-Against eigenray runs where they take every record and receiver by itself (beams in
-ray-centred coordinates): as many contributions as hits."""
+Beams in ray-centred coordinates against eigenray runs, whose gather takes every
+record and receiver by itself: as many contributions as hits."""
 import os
 
 import numpy as np
@@ -34,3 +34,29 @@ def test_raycen_beam_shift_without_loss(beam, tmp_path):
     hits, _ = run(s, root)
     assert st["evals"] == len(hits) > 0
     assert np.isnan(field).any()
+
+
+BOTTOM = [(-1.0, 3080.76622911), (3.41496, 2705.46346941), (3.98412, 2778.14218172), (5.1408, 2534.57457607),
+          (8.86788, 2793.5918653), (9.01476, 3286.31065653), (18.9, 3110.45643377)]
+SPEEDS = [1510.12842095, 1507.46967454, 1506.6479501, 1503.86137494, 1504.2264313, 1499.65926978, 1502.06426914,
+          1500.98318806, 1499.90210698, 1498.82102589, 1497.28074557, 1494.74556774, 1495.57778265, 1493.50869379,
+          1492.86381948, 1492.38595148, 1490.77940815, 1490.17237725, 1490.63031007, 1491.98978492, 1493.070866,
+          1494.18462547, 1495.23302816, 1496.27469847, 1497.99938253, 1498.73608054, 1498.78162588, 1501.16364204,
+          1501.61146881, 1504.72987296, 1504.72713614, 1504.96275789, 1506.88222121, 1507.22807957, 1508.20600113,
+          1509.28708221, 1512.70123607, 1510.99714923]
+
+
+@pytest.mark.parametrize("run_type", ["CG", "CB", "IG"])
+def test_infinite_spreading(run_type, tmp_path):
+    """A ray caught in a hollow of a curvilinear bottom, whose q grows until it is
+    infinite: such a beam reaches every depth of the range it passes, and since its
+    amplitude is 0 there and its width infinite, the whole column is not a number."""
+    r, z = np.array(BOTTOM).T
+    s = EnvSpec(title="inf", freq=50.0, ssp_type="S", top_bc="V", atten_unit="W", ssp_z=np.linspace(0.0, 4500.0, 38),
+                ssp_cp=np.array(SPEEDS), bot_bc="A", bot_hs=(4500.0, 1600.0, 500.0, 1.7, 0.6, 0.0), nsz=1,
+                sz=(121.62162162162163,), nrz=16, rz=(450.0, 4275.0), nrr=31, rr_km=(0.0, 18.0),
+                run_type=run_type + " RR S", nalpha=301, single_beam=True, isingle=74, alpha=(-80.0, 48.0), deltas=0.0,
+                box_z=4950.0, box_r_km=18.18, bty_r=r, bty_z=z, bty_type="CS")
+    field, _ = run(s, os.path.join(str(tmp_path), "e"))
+    bad = np.isnan(field[0])
+    assert bad.any() and np.array_equal(bad.any(axis=0), bad.all(axis=0))
