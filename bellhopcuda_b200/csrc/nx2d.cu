@@ -664,7 +664,8 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 sig = max(sig, fl);
             }
             int i0 = 0, i1 = E.nrz;
-            if(fabs(M.tx) > FLTD(0.50001)) {
+            // (a width that is not a number bounds nothing)
+            if(fabs(M.tx) > FLTD(0.50001) && sig == sig) {
                 const double rmax = (E.gaussian ? 4.0 : 1.0) * sig;
                 i0 = lower_f(E.rz, E.nrz, M.zlo - rmax);
                 i1 = upper_f(E.rz, E.nrz, M.zhi + rmax);

@@ -1,15 +1,17 @@
 """Beams whose spreading is not a finite number: a receiver test that compares with
 NaN or infinity keeps the receiver, and so must every rule that leaves out work.
 
-Beams in ray-centred coordinates against eigenray runs, whose gather takes every
-record and receiver by itself: as many contributions as hits."""
+Beams in ray-centred coordinates and N x 2-D beams against eigenray runs, whose
+gathers take every record and receiver by itself: as many contributions as hits."""
 import os
+import random
 
 import numpy as np
 import pytest
 
 import bellhopcuda_b200 as B
 from bellhopcuda_b200.envfile import EnvSpec, write_env
+from bellhopcuda_b200.envfile3d import env_text, grid_text, hex_ssp_text, write_files
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +62,40 @@ def test_infinite_spreading(run_type, tmp_path):
     field, _ = run(s, os.path.join(str(tmp_path), "e"))
     bad = np.isnan(field[0])
     assert bad.any() and np.array_equal(bad.any(axis=0), bad.all(axis=0))
+
+
+def hollows(seed, run_type):
+    """A curvilinear bottom of hollows under N x 2-D rays."""
+    r = random.Random(seed)
+    xy = np.linspace(-5.0, 5.0, r.choice([5, 7, 9]))
+    bty = np.array([[r.uniform(300.0, 980.0) for _ in xy] for _ in xy])
+    if r.random() < 0.5:
+        bty = np.repeat(bty[:, :1], len(xy), axis=1)
+    hexa = r.random() < 0.4
+    z = np.linspace(0.0, 1000.0, r.choice([2, 4, 9]))
+    c = 1500.0 - 10.0 * np.sin(z / 300.0)
+    beam = r.choice(["CG", "CB", "IG"])
+    f = {".bty": grid_text(xy, xy, np.round(bty, 2), "C")}
+    f[".env"] = env_text(title="hollows", freq=100.0, ssp_opt=("H" if hexa else r.choice("CSPN")) + r.choice("RV") + "W",
+                         depth=1000.0, ssp=list(zip(z, c)), bot=(r.choice("RV") + "~",), sx=[0.0], sy=[0.0], sz=[250.0],
+                         rz=None, rr_km=None, theta=[0.0, 60.0, 90.0, 180.0], run_type=(run_type or beam[0]) + beam[1] + "   2",
+                         alpha=(41, -80.0, 80.0), beta=(9, 0.0, 360.0), step=100.0, box_km=(4.2, 4.2), box_z=1100.0,
+                         nrz_range=(9, 100.0, 900.0), rr_range=(81, 0.0, 4.0))
+    if hexa:
+        h = np.linspace(-5.0, 5.0, 3)
+        X, _, Z = np.meshgrid(h, h, z, indexing="ij")
+        f[".ssp"] = hex_ssp_text(h, h, z, np.interp(Z, z, c) + (3.0 * np.sin(X) if r.random() < 0.5 else 0.0))
+    return f
+
+
+@pytest.mark.parametrize("seed", [20, 21, 7])
+def test_nx2d_spreading_not_a_number(seed, tmp_path):
+    """Rays caught in hollows: q grows until it is infinite, and then is not a number."""
+    root = os.path.join(str(tmp_path), "e")
+    with B.Tracer(precision=B.PREC_FP64) as t:
+        t.setup3d(write_files(hollows(seed, None), root)).run()
+        field, evals = t.field3d(), t.stats()["evals"]
+    with B.Tracer(precision=B.PREC_FP64) as t:
+        t.setup3d(write_files(hollows(seed, "E"), root)).run()
+        assert t.stats()["evals"] == evals
+    assert np.isnan(field).any()
