@@ -448,7 +448,7 @@ template<bool HEX> struct RayNWalk {
                 r2.taur = p0.taur + d0.r + d1.r;
                 r2.taui = p0.taui + d0.i + d1.i;
                 const V2<double> pq1p = scl2(-cnn1, qm), pq1q = scl2(b.c, pm);
-                r2.p = HEX ? p0.p : add2(add2(p0.p, scl2(k, pq0p)), scl2(hw1, pq1p));
+                r2.p = HEX ? pm : add2(add2(p0.p, scl2(k, pq0p)), scl2(hw1, pq1p));
                 r2.q = add2(add2(p0.q, scl2(k, pq0q)), scl2(hw1, pq1q));
                 r2.x = x;
                 r2.t = t;
@@ -462,7 +462,8 @@ template<bool HEX> struct RayNWalk {
             b = o;
             gb = grad(o);
             cnn1 = o.czz * t.x * t.x;
-            if(!HEX) pm = add2(p0.p, scl2(halfh, pq0p));
+            // HEX: czz is 0, and p changes by 0 q only (Ray2Seg::step)
+            pm = HEX ? mk2(fma(0.0, p0.q.x, p0.p.x), fma(0.0, p0.q.y, p0.p.y)) : add2(p0.p, scl2(halfh, pq0p));
             qm = add2(p0.q, scl2(halfh, pq0q));
             u = scl2(o.c, t);
         }

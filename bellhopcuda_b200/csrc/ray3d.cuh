@@ -225,6 +225,16 @@ template<bool HEX> struct Ray3Walk {
             const bool curved = !HEX && bent;
             M2 dp0, dp1;
             if(curved) dp0 = p_rate(p0, a);
+            // without a curvature p changes by 0 q only (Ray2Seg::step)
+            M2 ps = p0.p;
+            if(!curved) {
+#pragma unroll
+                for(int i = 0; i < 2; ++i) {
+                    const double z = fma(0.0, p0.q.m[0][i], 0.0 * p0.q.m[1][i]);
+                    ps.m[0][i] += z;
+                    ps.m[1][i] += z;
+                }
+            }
             const V3 u0 = scl3(c0, t0);
             const M2 dq0 = m2_scl(c0, p0.p);
             // Three passes over one copy of the crossing tests and of the
@@ -274,7 +284,7 @@ template<bool HEX> struct Ray3Walk {
                     r2.taui = p0.taui + d0.i + d1.i;
                     r2.phi = (p0.phi + k * f0) + hw1 * f1;
                     const M2 dq1 = m2_scl(b.c, r1.p);
-                    r2.p = curved ? m2_add(m2_add(p0.p, m2_scl(k, dp0)), m2_scl(hw1, dp1)) : p0.p;
+                    r2.p = curved ? m2_add(m2_add(p0.p, m2_scl(k, dp0)), m2_scl(hw1, dp1)) : ps;
                     r2.q = m2_add(m2_add(p0.q, m2_scl(k, dq0)), m2_scl(hw1, dq1));
                     r2.x = x;
                     r2.t = t;
@@ -289,7 +299,7 @@ template<bool HEX> struct Ray3Walk {
                 r1.x = x;
                 r1.t = t;
                 r1.phi = p0.phi + halfh * f0;
-                r1.p = curved ? m2_add(p0.p, m2_scl(halfh, dp0)) : p0.p;
+                r1.p = curved ? m2_add(p0.p, m2_scl(halfh, dp0)) : ps;
                 if(curved) r1.q = m2_add(p0.q, m2_scl(halfh, dq0));
                 f1 = phi_rate(t, o);
                 if(curved) dp1 = p_rate(r1, o);

@@ -2,7 +2,9 @@
 NaN or infinity keeps the receiver, and so must every rule that leaves out work.
 
 Beams in ray-centred coordinates and N x 2-D beams against eigenray runs, whose
-gathers take every record and receiver by itself: as many contributions as hits."""
+gathers take every record and receiver by itself: as many contributions as hits. The
+step over kept cells against the general step, which a batch of both kinds of ocean
+takes: contributions of the batch are the sum of those of its environments alone."""
 import os
 import random
 
@@ -99,3 +101,21 @@ def test_nx2d_spreading_not_a_number(seed, tmp_path):
         t.setup3d(write_files(hollows(seed, "E"), root)).run()
         assert t.stats()["evals"] == evals
     assert np.isnan(field).any()
+
+
+def test_nx2d_step_past_all_numbers(tmp_path):
+    """p changes by 0 q where the ocean has no depth curvature: nothing, until q is infinite."""
+    def evals(roots):
+        with B.Tracer(precision=B.PREC_FP64) as t:
+            for r in roots:
+                t.add_env3d(r)
+            t.run()
+            return t.stats()["steps"], t.stats()["evals"]
+    flat = env_text(title="flat", freq=100.0, ssp_opt="CVW", depth=1000.0, ssp=[(0.0, 1500.0), (1000.0, 1510.0)],
+                    bot=("R",), sx=[0.0], sy=[0.0], sz=[250.0], rz=None, rr_km=None, theta=[0.0, 90.0], run_type="CB   2",
+                    alpha=(5, -20.0, 20.0), beta=(9, 0.0, 360.0), step=100.0, box_km=(4.2, 4.2), box_z=1100.0,
+                    nrz_range=(9, 100.0, 900.0), rr_range=(81, 0.0, 4.0))
+    a = write_files(hollows(11, None), os.path.join(str(tmp_path), "a"))
+    b = write_files({".env": flat}, os.path.join(str(tmp_path), "b"))
+    (sa, ea), (sb, eb) = evals([a]), evals([b])
+    assert evals([a, b]) == (sa + sb, ea + eb)
