@@ -37,7 +37,7 @@ cudaError_t launch_arr_gather_nx(const void *, unsigned long long, const GroupDe
                                  uint64_t *, uint32_t *, unsigned long long, unsigned long long *, RunCounters *,
                                  ArrKeyBits, int, cudaStream_t);
 cudaError_t launch_influence_nx(const void *, unsigned long long, const GroupDev *, int, float2 *, RunCounters *, int,
-                                cudaStream_t);
+                                double, cudaStream_t);
 cudaError_t launch_scale_nx(float2 *, const GroupDev *, int, int, cudaStream_t);
 size_t nx_record_bytes();
 cudaError_t launch_trace3d(const GroupDev *, int, long long, long long, SegRec3 *, unsigned long long, RunCounters *,
@@ -582,8 +582,12 @@ void run_jobs(Run3 *r, long long j0, long long j1, cudaStream_t st, int sm_count
             return;
         }
         if(rc.err_bits == 0 && r->nx2d) {
+            double per_step = 0.0;
+            for(const auto &S : r->envs)
+                if(S.T.rr.size() > 1)
+                    per_step = std::max(per_step, S.T.deltas * (double)(S.T.rr.size() - 1) / (S.T.rr.back() - S.T.rr.front()));
             CK(launch_influence_nx(r->segs.p, nseg, (const GroupDev *)r->groups_d.p, (int)r->groups_h.size(),
-                                   (float2 *)r->field.p, ctr, sm_count * 16, st));
+                                   (float2 *)r->field.p, ctr, sm_count * 16, per_step, st));
         } else if(rc.err_bits == 0 && r->raycen) {
             int nzt = 1;   // (depth, bearing) pairs per record, the most of the batch
             for(const auto &S : r->envs) nzt = std::max(nzt, (int)(S.T.rz.size() * S.T.theta.size()));

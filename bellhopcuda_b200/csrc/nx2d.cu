@@ -622,13 +622,26 @@ template<int M> __global__ void __launch_bounds__(64) trace_nx_kernel(const Grou
 }
 
 // InfluenceGeoCore + ApplyContribution, 2-D Cartesian (src/influence.hpp:
-// 423-473, 897-1024). A warp stages 32 records; their (range, depth) items
-// inside the segments' depth windows (src/influence.hpp:1285-1292) are
-// flattened, so that every lane evaluates a receiver. Bound by the FP64 work
-// of the items and the field's 8-byte atomics. With one thread per record and
+// 423-473, 897-1024). A warp stages 32 records; their items inside the segments'
+// depth windows (src/influence.hpp:1285-1292), RUN ranges at a depth each, are
+// flattened, so that every lane evaluates receivers. Bound by the FP64 work of
+// the items and the field's 8-byte atomics. With one thread per record and
 // receiver depth, most of them outside the window, and the record read from
-// global memory by each, 12,996 rays x 501 x 101 receivers took 9.6 ms; now 1.5.
+// global memory by each, 12,996 rays x 501 x 101 receivers took 22.9 ms; this 3.9.
+//
+// Blocks of 32 records are too few for the chip where rays are few, and uneven
+// where receivers are dense, so a block's items are dealt to `parts` warps, for
+// about four units of work a warp. One warp a block against this, and one thread
+// per record and depth in brackets: 3 rays x 20000 x 2000 receivers 420 -> 1.8 ms
+// (1.6), 361 x 10001 x 2001 113 -> 39 (42), 1001 x 10001 x 1001 83 -> 54 (67).
+//
+// RUN is 1 or 8 (launch_influence_nx): an item's search for its record, its
+// division and the record's parts from shared memory are paid once a run, but a
+// step that brackets two or three ranges has no runs. RUN 1 and 8: 361 rays x
+// 10001 x 2001 receivers (50 ranges a step) 46 and 39 ms, 12,996 x 501 x 101
+// (2.5 a step) 3.9 and 4.4.
 constexpr int WARPSN = 4;
+template<int RUN>
 __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<double> *__restrict__ segs,
                                                                    unsigned long long cap,
                                                                    const GroupDev *__restrict__ groups, int ngroups,
@@ -642,9 +655,12 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
     const unsigned long long nseg = min(__ldcg(&ctr->nseg), cap);
     const unsigned long long nchunks = (nseg + 31) / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned int nwarps = gridDim.x * WARPSN;
+    const unsigned int parts = nchunks < 4 * nwarps ? 4 * nwarps / max((unsigned int)nchunks, 1u) : 1u;
     unsigned int evals = 0;
-    for(unsigned long long ch = blockIdx.x * (unsigned long long)WARPSN + w; ch < nchunks;
-        ch += (unsigned long long)gridDim.x * WARPSN) {
+    for(unsigned long long u = blockIdx.x * (unsigned long long)WARPSN + w; u < nchunks * parts; u += nwarps) {
+        const unsigned long long ch = u / parts;
+        const unsigned int part = (unsigned int)(u - ch * parts);
         const int nvalid = (int)min(32ull, nseg - ch * 32);
         {
             const int words = sizeof(SegRec<double>) / 16;
@@ -672,7 +688,7 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 i1 = upper_f(E.rz, E.nrz, M.zhi + rmax);
             }
             if(i1 > i0) {
-                n = (M.ir_hi - M.ir_lo + 1) * (i1 - i0);
+                n = (M.ir_hi - M.ir_lo + RUN) / RUN * (i1 - i0);
                 const Job3 J = job_indices3(E, (int)((long long)M.job - G.job_base));
                 s_row[w][lane] = G.field_base
                     + ((((long long)J.isz * E.nsx + J.isx) * E.nsy + J.isy) * E.ntheta + J.ibeta) * E.nrz * E.nrr;
@@ -692,47 +708,54 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
         s_incl[w][lane] = incl;
         __syncwarp();
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        for(int it = lane; it < total; it += 32) {
+        for(long long at = 32 * part + lane; at < total; at += 32 * parts) {
+            const int it = (int)at;
             int lo = 0, hi = 31;   // first record j with incl[j] > it
             while(lo < hi) {
                 const int mid = (lo + hi) >> 1;
                 if(s_incl[w][mid] > it) hi = mid; else lo = mid + 1;
             }
             const int j = lo, local = it - (j ? s_incl[w][j - 1] : 0);
-            const int niz = s_niz[w][j], col = local / niz, iz = s_iz0[w][j] + local - col * niz;
+            const int niz = s_niz[w][j], run = local / niz, iz = s_iz0[w][j] + local - run * niz;
             const SegRec<double> &S = s_rec[w][j];
             const Env3Dev &E = *s_env[w][j];
             const bool gauss = E.gaussian != 0, coherent = E.coherent != 0;
-            const int ir = S.ir_lo + col;
-            const double dz = (double)E.rz[iz] - S.x0z, dr = E.rr[ir] - S.x0r;
-            const double s = quot_rn(dr * S.tx + dz * S.tz, S.rlen, s_rcp[w][j]);
-            const double n1 = fabs(dz * S.tx - dr * S.tz);
-            const double qF = S.q0 + s * S.dq;
-            double sigma = fabs(qF * S.rcp_q0);
-            const double sig0 = sigma;
-            if(gauss) sigma = max(sigma, s_fl[w][j]);
-            if(n1 >= (gauss ? 4.0 : 1.0) * sigma) continue;
-            const double cnst = S.cnst_num / sqrt(fabs(qF));
-            const double wgt = gauss ? exp(FLTD(-0.5) * (n1 / sigma) * (n1 / sigma)) * (sig0 / sigma)
-                                     : (sigma - n1) / sigma;
-            const bool caustic = (qF <= 0.0 && S.q0 > 0.0) || (qF >= 0.0 && S.q0 < 0.0);
-            const double ph = caustic ? S.phase_b : S.phase_a;
+            const double dz = (double)E.rz[iz] - S.x0z, fl = s_fl[w][j], rcp = s_rcp[w][j];
             const double omega = FLTD(2.0) * BHCB_PI * E.freq0;
-            const double di = S.tau0i + s * S.dtaui;
-            float2 v;
-            if(coherent) {
-                const double amp = cnst * wgt * exp(omega * di);
-                double sn, cs;
-                sincos(reduce_2pi(omega * (S.tau0r + s * S.dtaur) - ph), &sn, &cs);
-                v = make_float2((float)(amp * cs), (float)(-amp * sn));
-            } else {
-                double vv = cnst * exp(omega * di);
-                vv = vv * vv * wgt;
-                if(gauss) vv *= sqrt(FLTD(2.0) * BHCB_PI);
-                v = make_float2((float)vv, 0.f);
-            }
-            atomicAdd(field + s_row[w][j] + (long long)iz * E.nrr + ir, v);
-            ++evals;
+            float2 *row = field + s_row[w][j] + (long long)iz * E.nrr;
+            int ir = S.ir_lo + run * RUN;
+            const int ir1 = min(ir + RUN - 1, S.ir_hi);
+#pragma unroll 1
+            do {
+                const double dr = E.rr[ir] - S.x0r;
+                const double s = quot_rn(dr * S.tx + dz * S.tz, S.rlen, rcp);
+                const double n1 = fabs(dz * S.tx - dr * S.tz);
+                const double qF = S.q0 + s * S.dq;
+                double sigma = fabs(qF * S.rcp_q0);
+                const double sig0 = sigma;
+                if(gauss) sigma = max(sigma, fl);
+                if(n1 >= (gauss ? 4.0 : 1.0) * sigma) continue;
+                const double cnst = S.cnst_num / sqrt(fabs(qF));
+                const double wgt = gauss ? exp(FLTD(-0.5) * (n1 / sigma) * (n1 / sigma)) * (sig0 / sigma)
+                                         : (sigma - n1) / sigma;
+                const bool caustic = (qF <= 0.0 && S.q0 > 0.0) || (qF >= 0.0 && S.q0 < 0.0);
+                const double ph = caustic ? S.phase_b : S.phase_a;
+                const double di = S.tau0i + s * S.dtaui;
+                float2 v;
+                if(coherent) {
+                    const double amp = cnst * wgt * exp(omega * di);
+                    double sn, cs;
+                    sincos(reduce_2pi(omega * (S.tau0r + s * S.dtaur) - ph), &sn, &cs);
+                    v = make_float2((float)(amp * cs), (float)(-amp * sn));
+                } else {
+                    double vv = cnst * exp(omega * di);
+                    vv = vv * vv * wgt;
+                    if(gauss) vv *= sqrt(FLTD(2.0) * BHCB_PI);
+                    v = make_float2((float)vv, 0.f);
+                }
+                atomicAdd(row + ir, v);
+                ++evals;
+            } while(RUN > 1 && ++ir <= ir1);
         }
         __syncwarp();
     }
@@ -985,10 +1008,12 @@ cudaError_t launch_arr_gather_nx(const void *segs, unsigned long long nseg, cons
     return cudaGetLastError();
 }
 
+// ranges_per_step: receiver ranges in a step of the densest environment
 cudaError_t launch_influence_nx(const void *segs, unsigned long long cap, const GroupDev *groups, int ngroups,
-                                float2 *field, RunCounters *ctr, int grid, cudaStream_t st)
+                                float2 *field, RunCounters *ctr, int grid, double ranges_per_step, cudaStream_t st)
 {
-    influence_nx_kernel<<<grid, 32 * WARPSN, 0, st>>>((const SegRec<double> *)segs, cap, groups, ngroups, field, ctr);
+    auto k = ranges_per_step >= 16.0 ? influence_nx_kernel<8> : influence_nx_kernel<1>;
+    k<<<grid, 32 * WARPSN, 0, st>>>((const SegRec<double> *)segs, cap, groups, ngroups, field, ctr);
     return cudaGetLastError();
 }
 
