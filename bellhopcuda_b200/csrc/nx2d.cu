@@ -633,7 +633,7 @@ template<int M> __global__ void __launch_bounds__(64) trace_nx_kernel(const Grou
 // where receivers are dense, so a block's items are dealt to `parts` warps, for
 // about four units of work a warp. One warp a block against this, and one thread
 // per record and depth in brackets: 3 rays x 20000 x 2000 receivers 420 -> 1.8 ms
-// (1.6), 361 x 10001 x 2001 113 -> 39 (42), 1001 x 10001 x 1001 83 -> 54 (67).
+// (1.6), 361 x 10001 x 2001 113 -> 39 (42), 1001 x 10001 x 1001 83 -> 58 (67).
 //
 // RUN is 1 or 8 (launch_influence_nx): an item's search for its record, its
 // division and the record's parts from shared memory are paid once a run, but a
@@ -641,6 +641,7 @@ template<int M> __global__ void __launch_bounds__(64) trace_nx_kernel(const Grou
 // 10001 x 2001 receivers (50 ranges a step) 46 and 39 ms, 12,996 x 501 x 101
 // (2.5 a step) 3.9 and 4.4.
 constexpr int WARPSN = 4;
+constexpr int NX_PASS = 1 << 25;   // items of one record in a pass
 template<int RUN>
 __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<double> *__restrict__ segs,
                                                                    unsigned long long cap,
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
             for(int k = lane; k < nvalid * words; k += 32) dst[k] = __ldcs(src + k);
         }
         __syncwarp();
-        int n = 0;
+        long long items = 0;
         const SegRec<double> &M = s_rec[w][lane];
         if(lane < nvalid && M.job >= 0) {
             const GroupDev &G = groups[find_group(groups, ngroups, M.job)];
@@ -688,7 +689,7 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 i1 = upper_f(E.rz, E.nrz, M.zhi + rmax);
             }
             if(i1 > i0) {
-                n = (M.ir_hi - M.ir_lo + RUN) / RUN * (i1 - i0);
+                items = (long long)((M.ir_hi - M.ir_lo + RUN) / RUN) * (i1 - i0);
                 const Job3 J = job_indices3(E, (int)((long long)M.job - G.job_base));
                 s_row[w][lane] = G.field_base
                     + ((((long long)J.isz * E.nsx + J.isx) * E.nsy + J.isy) * E.ntheta + J.ibeta) * E.nrz * E.nrr;
@@ -699,7 +700,11 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 s_rcp[w][lane] = rcp_ulp(M.rlen);
             }
         }
-        int incl = n;
+        // passes of at most NX_PASS items of every record, so that the sums of 32 fit an int
+        const unsigned int passes = __reduce_max_sync(0xffffffffu, (unsigned int)((items + NX_PASS - 1) / NX_PASS));
+        for(unsigned int pass = 0; pass < passes; ++pass) {
+        const long long first = (long long)pass * NX_PASS;
+        int incl = (int)min(max(items - first, 0LL), (long long)NX_PASS);
 #pragma unroll
         for(int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -716,7 +721,8 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 if(s_incl[w][mid] > it) hi = mid; else lo = mid + 1;
             }
             const int j = lo, local = it - (j ? s_incl[w][j - 1] : 0);
-            const int niz = s_niz[w][j], run = local / niz, iz = s_iz0[w][j] + local - run * niz;
+            const int niz = s_niz[w][j], run = pass ? (int)((first + local) / niz) : local / niz;
+            const int iz = s_iz0[w][j] + (int)(first + local - (long long)run * niz);
             const SegRec<double> &S = s_rec[w][j];
             const Env3Dev &E = *s_env[w][j];
             const bool gauss = E.gaussian != 0, coherent = E.coherent != 0;
@@ -756,6 +762,8 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 atomicAdd(row + ir, v);
                 ++evals;
             } while(RUN > 1 && ++ir <= ir1);
+        }
+        __syncwarp();
         }
         __syncwarp();
     }

@@ -34,3 +34,24 @@ def test_contributions(beam, nalpha, nrr, nrz, tmp_path):
     at = np.zeros(field.shape, bool)
     at[hits["isz"], hits["itheta"], hits["iz"], hits["ir"]] = True
     assert not np.any((field != 0) & ~at)
+
+
+def test_more_items_than_a_pass(tmp_path):
+    """15 ranges a step at 2.4 million depths: more than 2^25 items of a record, which take
+    two passes. Depths are exact in FP32, so the two halves of the grid, one pass each,
+    hold the same receivers: their contributions sum to the whole grid's."""
+    def evals(i0, n):
+        text = env_text(title="deep", freq=120.0, ssp_opt="CVW", depth=1000.0, ssp=[(0.0, 1500.0), (1000.0, 1510.0)],
+                        bot=("A", 1650.0, 1.6, 0.5), sx=[0.0], sy=[0.0], sz=[250.0], rz=None, rr_km=None, theta=[0.0],
+                        run_type="CB   2", alpha=(2, -3.0, 4.0), beta=(9, 0.0, 360.0), step=5000.0, box_km=(10.2, 10.2),
+                        box_z=1100.0, nrz_range=(n, 256.0 + i0 / 8192.0, 256.0 + (i0 + n - 1) / 8192.0),
+                        rr_range=(31, 0.0, 10.0))
+        text = text.replace("%g %g /" % (256.0 + i0 / 8192.0, 256.0 + (i0 + n - 1) / 8192.0),
+                            "%.13f %.13f /" % (256.0 + i0 / 8192.0, 256.0 + (i0 + n - 1) / 8192.0))
+        with B.Tracer(precision=B.PREC_FP64) as t:
+            t.setup3d(write_files({".env": text}, os.path.join(str(tmp_path), "e"))).run()
+            return t.stats()["evals"]
+    half = 1 << 20
+    n = 2400000
+    total = evals(0, n)
+    assert total == evals(0, half) + evals(half, half) + evals(2 * half, n - 2 * half) > 15 * half
