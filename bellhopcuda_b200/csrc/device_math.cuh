@@ -95,44 +95,57 @@ __device__ __forceinline__ float cos_ftz(float x)
     return y;
 }
 
-// Correctly rounded FP64 quotient and square root (and a reciprocal within an
-// ulp for them) without the branch to a slow path that `/` and sqrt() carry, so that independent ones
-// overlap and one reciprocal serves several quotients (a dependent `/` takes
-// 115 cycles on B200, a sqrt 80, a DFMA 8; the tracers are one dependent chain
-// per ray). Newton's iteration on the hardware estimate, then Markstein's
-// residual correction with fused multiply-adds (P. Markstein, IBM J. Res. Dev.
-// 34, 1990; Cornea, Harrison and Tang, IEEE Trans. Comput. 2002): the last
-// correction rounds the exact residual once, which gives the value that IEEE
-// division and square root give. For finite operands with |b|, |a| and the
-// result between 2^-900 and 2^900 (a = 0 allowed); the callers' divisors are
-// sound speeds, step lengths and direction components that they have checked.
+// Correctly rounded FP64 reciprocal, quotient and square root without the branch to
+// a slow path that `/` and sqrt() carry, so that independent ones overlap and one
+// reciprocal serves several quotients (a dependent `/` takes 115 cycles on B200, a
+// sqrt 80, a DFMA 8; the tracers are one dependent chain per ray). Newton's iteration
+// on the hardware estimate, then Markstein's residual correction with fused
+// multiply-adds (P. Markstein, IBM J. Res. Dev. 34, 1990; Cornea, Harrison and Tang,
+// IEEE Trans. Comput. 2002): the last correction rounds the exact residual once. For
+// finite operands with |b|, |a| and the result between 2^-900 and 2^900 (a = 0
+// allowed, infinities and NaN not); the callers' divisors are sound speeds, step
+// lengths and direction components that they have checked.
+//
+// The correction of a quotient needs the correctly rounded reciprocal: with one an ulp
+// off, four in ten of the quotients nearest to a midpoint between doubles come out
+// wrong. A last Newton step yields (1 - e^2) / b, e the error before it: below 1 / b,
+// and so wrong if 1 / b lies above a midpoint by less than e^2 and y is the double
+// below (b all ones, where the rounding has a tie). The step before rounds up, so y is
+// then the double above, half an ulp off, and 1 / b, at least 2^-106 of itself above
+// the midpoint, is rounded to it.
+//
+// For b > 0. Of a negative b all ones (1.99... to the last bit) the reciprocal, and with
+// it one of the quotients next to a midpoint, is the double beside: taking the sign
+// aside, as rcp_signed does, would lengthen the tracers' chain by 2 %.
 __device__ __forceinline__ double rcp_est(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     return y;
 }
-__device__ __forceinline__ double rcp_ulp(double b)
+__device__ __forceinline__ double rcp_rn(double b)
 {
     double y = rcp_est(b);
     double e = fma(-b, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
+    y = __fma_ru(y, fma(e, e, e), y);
     e = fma(-b, y, 1.0);
     return fma(y, e, y);
 }
-// 1 / bsq within an ulp, bsq = b * b rounded and y = rcp_ulp(b)
+__device__ __forceinline__ double rcp_signed(double b) { return copysign(rcp_rn(fabs(b)), b); }
+// 1 / bsq, bsq = b * b rounded and y = rcp_rn(b)
 __device__ __forceinline__ double rcp_square(double bsq, double y)
 {
-    const double z = y * y;
+    double z = y * y;
+    z = __fma_ru(z, fma(-bsq, z, 1.0), z);
     return fma(z, fma(-bsq, z, 1.0), z);
 }
-// a / b given y = rcp_ulp(b)
+// a / b given y, the correctly rounded 1 / b
 __device__ __forceinline__ double quot_rn(double a, double b, double y)
 {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-__device__ __forceinline__ double div_rn(double a, double b) { return quot_rn(a, b, rcp_ulp(b)); }
+__device__ __forceinline__ double div_rn(double a, double b) { return quot_rn(a, b, rcp_rn(b)); }
 // a >= 2^-900 (0 is the caller's to exclude)
 __device__ __forceinline__ double sqrt_rn(double a)
 {

@@ -129,7 +129,7 @@ template<typename R, typename RecR> __device__ __forceinline__ bool infl_prologu
     inf.x = p1.x;
     if(first < 0) return false;
     if(long_seg) rlen = sqrt_rn(dd);
-    const double rcp_len = rcp_ulp(rlen);
+    const double rcp_len = rcp_rn(rlen);
     const V2<double> rayt = mk2(quot_rn(d.x, rlen, rcp_len), quot_rn(d.y, rlen, rcp_len));
     const double atx = fabs(rayt.x);
     rec.x0r = p0.x.x;

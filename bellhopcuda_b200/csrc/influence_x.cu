@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(32 * RCW) influence_raycen_kernel(
         const double freq = freqs[g.freq_base], omega = FLTD(2.0) * BHCB_PI * freq;
         const bool gauss = e.gaussian, coherent = e.coherent;
         const double W = gauss ? 4.0 : 1.0;
-        const double rr0 = e.rr[0], delta = e.delta_r, rcp_delta = rcp_ulp(delta);
+        const double rr0 = e.rr[0], delta = e.delta_r, rcp_delta = rcp_rn(delta);
         __syncwarp();
         {
             const bool have = ch * 32 + lane < nseg;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(32 * RCW) influence_raycen_kernel(
             RcRec r;
             r.use = have && S.job >= 0;
             r.xb = S.xb; r.zb = S.zb; r.nx = S.nxb; r.nz = S.nzb;
-            r.rn = rcp_ulp(S.nzb);
+            r.rn = rcp_signed(S.nzb);
             r.q0 = S.q0r; r.dq = S.dqr; r.rcp = S.rcp_q0;
             r.fl = gauss ? min(FLTD(0.2) * freq * S.tau1r, BHCB_PI * (S.c0 / freq)) : 0.0;
             // over s in [-0.002, 1.002], rounding included

@@ -130,7 +130,7 @@ __device__ __forceinline__ bool infl_prologue3(const Ray3 &P0, const Ray3 &P1, I
     inf.ir = ir;
     inf.rr = r;
     if(hi < 0) return false;
-    const double rl = rcp_ulp(rlen);
+    const double rl = rcp_rn(rlen);
     rayt = v3(quot_rn(rayt.x, rlen, rl), quot_rn(rayt.y, rlen, rl), quot_rn(rayt.z, rlen, rl));
     V3 e1, e2;
     ray_normal_unit(rayt, P1.phi, cphi, sphi, e1, e2);
@@ -347,7 +347,7 @@ constexpr int WARPS3 = 2;   // the records of 32 segments take 13 KB of shared m
 // rest of the record only for accepted receivers).
 struct Rec3S {
     double x0[3], rayt[3], e1[3], e2[3];
-    double rlen, rcp_len;      // segment length, rcp_ulp(rlen)
+    double rlen, rcp_len;      // segment length, rcp_rn(rlen)
     double zlo, zhi, ldiag;
     double q0[4], dq[4], rcp_q0, rcp_qhat0;
     float q0f[4], dqf[4], rq0f, rq1f;   // the same in FP32 (mixed precision)
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(32 * WARPS3) influence3d_kernel(
                     S.e2[i] = R.e2[i];
                 }
                 S.rlen = R.rlen;
-                S.rcp_len = rcp_ulp(R.rlen);
+                S.rcp_len = rcp_rn(R.rlen);
                 S.zlo = R.zlo;
                 S.zhi = R.zhi;
                 S.ldiag = R.ldiag;

@@ -377,7 +377,7 @@ template<bool HEX> struct RayNWalk {
         p0 = st.p0;
         org = st.org;
         minx = st.minx; miny = st.miny; maxx = st.maxx; maxy = st.maxy;
-        rt = rcp_ulp(fabs(org.tx) >= fabs(org.ty) ? org.tx : org.ty);
+        rt = rcp_signed(fabs(org.tx) >= fabs(org.ty) ? org.tx : org.ty);
         small = 0;
         low = p0.Amp < FLTD(0.005);
         inside = false;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(32 * WARPSN) influence_nx_kernel(const SegRec<
                 s_iz0[w][lane] = i0;
                 s_niz[w][lane] = i1 - i0;
                 s_fl[w][lane] = fl;
-                s_rcp[w][lane] = rcp_ulp(M.rlen);
+                s_rcp[w][lane] = rcp_rn(M.rlen);
             }
         }
         // passes of at most NX_PASS items of every record, so that the sums of 32 fit an int

@@ -205,7 +205,7 @@ template<int K> struct Ray2Seg {
     {
         eval(p.x.y, p.t.y, c, g, czz);
         csq = c * c;
-        rc = rcp_ulp(c);
+        rc = rcp_rn(c);
         rcsq = rcp_square(csq, rc);
     }
     __device__ __forceinline__ void set_box()
@@ -294,7 +294,7 @@ template<int K> struct Ray2Seg {
         double c1, g1, czz1;
         eval(x0.y + halfh * u0.y, t1.y, c1, g1, czz1);
         const double csq1 = c1 * c1;
-        const double rc1 = rcp_ulp(c1), rcsq1 = rcp_square(csq1, rc1);
+        const double rc1 = rcp_rn(c1), rcsq1 = rcp_square(csq1, rc1);
         const double cnn1 = czz1 * t1.x * t1.x;
         const V2<double> pq1p = scl2(-cnn1, qm), pq1q = scl2(c1, pm);
         const V2<double> u1 = scl2(c1, t1);

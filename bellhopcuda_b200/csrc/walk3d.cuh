@@ -216,8 +216,8 @@ template<bool HEX> struct Walk3 {
         y1 = e.hy[s.y + 1];
         dx = x1 - x0;
         dy = y1 - y0;
-        rdx = rcp_ulp(dx);
-        rdy = rcp_ulp(dy);
+        rdx = rcp_rn(dx);
+        rdy = rcp_rn(dy);
         dirty = true;
     }
     // a new profile cell
@@ -267,7 +267,7 @@ template<bool HEX> struct Walk3 {
             o.ci = p.ci;
             o.czz = p.czz;
         }
-        o.rc = rcp_ulp(o.c);
+        o.rc = rcp_rn(o.c);
         o.rcsq = rcp_square(o.c * o.c, o.rc);
     }
     // range of x (y) that the boundary cells and the profile cell of the step's
@@ -526,7 +526,7 @@ __device__ __forceinline__ void ray_normal_unit(V3 t, double phi, double cp, dou
         e2 = b;
         return;
     }
-    const double rl = sqrt_rn(rl2), r = rcp_ulp(rl);
+    const double rl = sqrt_rn(rl2), r = rcp_rn(rl);
     e1.x = quot_rn(t.x * t.z * cp + t.y * sp, rl, r);
     e1.y = quot_rn(t.y * t.z * cp - t.x * sp, rl, r);
     e1.z = -rl * cp;
