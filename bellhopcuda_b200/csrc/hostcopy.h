@@ -30,12 +30,8 @@ public:
     // copy.
     cudaError_t copy(void *dst, const void *src, size_t bytes, cudaStream_t st)
     {
-        cudaPointerAttributes at{};
-        if(bytes < MIN_BYTES || cudaPointerGetAttributes(&at, dst) != cudaSuccess
-           || at.type != cudaMemoryTypeUnregistered || !prepare()) {
-            cudaGetLastError();
+        if(bytes < MIN_BYTES || !pageable(dst) || !prepare())
             return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
-        }
         int device = 0;
         cudaError_t err = cudaGetDevice(&device);
         if(err != cudaSuccess) return err;
@@ -108,6 +104,15 @@ private:
     cudaEvent_t ev_[SLOTS] = {};
     std::atomic<long long> done_[SLOTS];   // last chunk copied out of each slot
 
+    // Errors of the two probes below are taken back, so that the caller does not find
+    // them; an error from before the copy is left for whoever asks for it.
+    static bool pageable(const void *p)
+    {
+        cudaPointerAttributes at{};
+        if(cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        return false;
+    }
     bool prepare()
     {
         if(ring_) return true;
@@ -115,7 +120,10 @@ private:
         bool ok = cudaHostAlloc(&p, CHUNK * SLOTS, cudaHostAllocDefault) == cudaSuccess;
         ring_ = ok ? (char *)p : nullptr;
         for(auto &e : ev_) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-        if(!ok) release();
+        if(!ok) {
+            cudaGetLastError();
+            release();
+        }
         return ok;
     }
 };
