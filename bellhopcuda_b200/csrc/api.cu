@@ -696,10 +696,12 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
         return;
     }
     int tblock = c->trace_block;
+    const int kind = seg_kind(c, g0, g1);
     unsigned int stage_bytes = 0;   // tables of the launched groups that fit the staging budget
     for(int g = g0; g < g1; ++g) {
         size_t off[ST_COUNT];
-        stage_bytes = std::max<unsigned int>(stage_bytes, (unsigned int)stage_plan(c->envdev_h[g], c->stage_cap, off));
+        const size_t bytes = stage_plan(c->envdev_h[g], kind != 0, c->stage_cap, off);
+        stage_bytes = std::max(stage_bytes, (unsigned int)bytes);
     }
     const int warps = tblock / 32;
     const int tgrid = std::max(1, std::min((blk1 - blk0 + warps - 1) / warps, c->sm_count * 32));
@@ -721,10 +723,10 @@ void do_launch_range(bhcb_ctx *c, int g0, int g1, bool clear, bool host_driven)
     }
     if(fp64)
         CK(launch_trace<double>(G, ng, blk1, c->segs.p, c->seg_cap, ctr, jobc, blk, tgrid, tblock,
-                                c->stream, stage_bytes, seg_kind(c, g0, g1)));
+                                c->stream, stage_bytes, kind));
     else
         CK(launch_trace<float>(G, ng, blk1, c->segs.p, c->seg_cap, ctr, jobc, blk, tgrid, tblock,
-                               c->stream, stage_bytes, seg_kind(c, g0, g1)));
+                               c->stream, stage_bytes, kind));
     CK(record_event(c, 1, c->stream));
     if(c->mode != MODE_TL) return;   // arrivals / hits: run_arrivals after the trace
     if(ovl) {
@@ -825,20 +827,21 @@ void launch_pipelined(bhcb_ctx *c)
     CK(cudaMemsetAsync(acc, 0, acc_bytes, A));
     const GroupDev *G = (const GroupDev *)c->groups_d.p;
     const int ng = (int)c->groups_h.size();
-    const int tblock = c->trace_block;
+    const int tblock = c->trace_block, kind = seg_kind(c, 0, ng);
     unsigned int stage_bytes = 0;
     for(int g = 0; g < ng; ++g) {
         size_t off[ST_COUNT];
-        stage_bytes = std::max<unsigned int>(stage_bytes, (unsigned int)stage_plan(c->envdev_h[g], c->stage_cap, off));
+        const size_t bytes = stage_plan(c->envdev_h[g], kind != 0, c->stage_cap, off);
+        stage_bytes = std::max(stage_bytes, (unsigned int)bytes);
     }
     const int warps = tblock / 32;
     const int tgrid = std::max(1, std::min((c->nblocks + warps - 1) / warps, c->sm_count * 32));
     if(fp64)
         CK(launch_trace<double>(G, ng, c->nblocks, segs, c->seg_cap, ctr, jobc, nullptr, tgrid, tblock, A,
-                                stage_bytes, seg_kind(c, 0, ng)));
+                                stage_bytes, kind));
     else
         CK(launch_trace<float>(G, ng, c->nblocks, segs, c->seg_cap, ctr, jobc, nullptr, tgrid, tblock, A,
-                               stage_bytes, seg_kind(c, 0, ng)));
+                               stage_bytes, kind));
     CK(cudaEventRecord(ev[1], A));
     CK(cudaStreamWaitEvent(Bs, ev[1], 0));
     CK(cudaEventRecord(ev[2], Bs));

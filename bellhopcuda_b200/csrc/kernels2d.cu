@@ -45,7 +45,8 @@ template<typename R, typename RecR, int K> __global__ void __launch_bounds__(64)
     const int lane = (int)(threadIdx.x & 31);
     const int hint = min(end_block - 1, groups[0].blk_base + (int)(blockIdx.x * (blockDim.x >> 5)));
     const int gs = find_block_group(groups, ngroups, hint);
-    const bool staged = stage_budget > 0 && stage_env_tables(groups[gs].env, s_env, s_tab, stage_budget, &s_bar, ctr);
+    const bool staged = stage_budget > 0
+        && stage_env_tables(groups[gs].env, K != 0, s_env, s_tab, stage_budget, &s_bar, ctr);
     for(;;) {
         __syncwarp();
         unsigned long long taken = 0;

@@ -21,8 +21,8 @@
 namespace bhcb {
 
 // in the order of their reads per step: SSP nodes and coefficients (three
-// evaluations per step; the packed segments in their place where there are
-// any), boundary nodes (segment checks), receiver ranges
+// evaluations per step; the packed segments in their place where the launch's
+// step reads those), boundary nodes (segment checks), receiver ranges
 enum StageTable : int { ST_SEG, ST_Z, ST_C, ST_CZ, ST_COEF, ST_N2, ST_N2Z, ST_RHO, ST_QR, ST_QC, ST_QCZ, ST_BTOP, ST_BBOT,
                         ST_RR, ST_COUNT };
 
@@ -32,24 +32,26 @@ __host__ __device__ inline size_t round16(size_t b) { return (b + 15) & ~size_t(
 constexpr unsigned int STAGE_MAX_BYTES = 64u * 1024u;
 constexpr unsigned int STAGE_DEFAULT_BYTES = 32u * 1024u;
 
-// bytes of each table the step of this environment's SSP type reads (0: not read)
-__host__ __device__ inline void stage_table_bytes(const EnvDev &e, size_t b[ST_COUNT])
+// bytes of each table the step of this environment's SSP type reads (0: not read).
+// packed: the launch's step is the one over packed segments; a batch of several
+// profile types takes the general one, for environments that have them too
+__host__ __device__ inline void stage_table_bytes(const EnvDev &e, bool packed, size_t b[ST_COUNT])
 {
     for(int k = 0; k < ST_COUNT; ++k) b[k] = 0;
     const size_t n = (size_t)e.nssp;
     const int t = e.ssp_type;
-    if(e.has_seg) {
+    if(packed) {
         // the step reads the packed segments; nodes and coefficients only at reflections
         b[ST_SEG] = (n - 1) * sizeof(SspSeg);
     } else if(t != SSP_ANALYTIC) {
         b[ST_Z] = n * 8;
         b[ST_RHO] = n * 8;   // reflections (and N2-linear) interpolate the density
     }
-    if((t == SSP_CLINEAR && !e.has_seg) || t == SSP_QUAD) {
+    if((t == SSP_CLINEAR && !packed) || t == SSP_QUAD) {
         b[ST_C] = 2 * n * 8;
         if(t == SSP_CLINEAR) b[ST_CZ] = 2 * n * 8;
     }
-    if((t == SSP_CUBIC || t == SSP_PCHIP) && !e.has_seg) b[ST_COEF] = 8 * n * 8;
+    if((t == SSP_CUBIC || t == SSP_PCHIP) && !packed) b[ST_COEF] = 8 * n * 8;
     if(t == SSP_N2LINEAR) {
         b[ST_N2] = 2 * n * 8;
         b[ST_N2Z] = 2 * n * 8;
@@ -66,10 +68,10 @@ __host__ __device__ inline void stage_table_bytes(const EnvDev &e, size_t b[ST_C
 
 // shared-memory offsets of the tables that fit in budget (SIZE_MAX: stays in
 // global memory); returns the bytes used
-__host__ __device__ inline size_t stage_plan(const EnvDev &e, size_t budget, size_t off[ST_COUNT])
+__host__ __device__ inline size_t stage_plan(const EnvDev &e, bool packed, size_t budget, size_t off[ST_COUNT])
 {
     size_t b[ST_COUNT];
-    stage_table_bytes(e, b);
+    stage_table_bytes(e, packed, b);
     size_t used = 0;
     for(int k = 0; k < ST_COUNT; ++k) {
         off[k] = (size_t)-1;
@@ -113,15 +115,15 @@ constexpr unsigned STAGE_WAIT_LIMIT = 1u << 22;
 // the tables, rewrites s_env's pointers to the staged copies and issues the
 // bulk copies; all threads then wait for them. Returns false (and sets
 // ERR_STAGE_WAIT) when the wait ran out: the caller then reads global memory.
-__device__ __forceinline__ bool stage_env_tables(const EnvDev *src, EnvDev &s_env, unsigned char *s_tab,
-                                                 size_t budget, uint64_t *s_bar, RunCounters *ctr)
+__device__ __forceinline__ bool stage_env_tables(const EnvDev *src, bool packed, EnvDev &s_env,
+                                                 unsigned char *s_tab, size_t budget, uint64_t *s_bar, RunCounters *ctr)
 {
     using namespace stage_detail;
     if(threadIdx.x == 0) {
         s_env = *src;
         size_t off[ST_COUNT], b[ST_COUNT];
-        const size_t total = stage_plan(s_env, budget, off);
-        stage_table_bytes(s_env, b);
+        const size_t total = stage_plan(s_env, packed, budget, off);
+        stage_table_bytes(s_env, packed, b);
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(s_bar)), "r"(1u) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
