@@ -992,7 +992,7 @@ cudaError_t launch_trace_nx(const GroupDev *groups, int ngroups, long long njobs
                             unsigned long long cap, RunCounters *ctr, unsigned long long *job_counter, int sm_count,
                             int kind, cudaStream_t st)
 {
-    const int lanes = lanes3(njobs, sm_count);
+    const int lanes = lanes3(njobs, sm_count, kind != 0);
     const long long warps = (njobs + lanes - 1) / lanes;
     const int grid = (int)std::max(1LL, std::min<long long>((warps + 1) / 2, (long long)sm_count * 16));
     auto k = kind == 1 ? trace_nx_kernel<1> : kind == 2 ? trace_nx_kernel<2> : trace_nx_kernel<0>;

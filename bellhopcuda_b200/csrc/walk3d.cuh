@@ -24,12 +24,17 @@
 
 namespace bhcb {
 
-// Rays per warp of a 3-D or Nx2D trace: as few as keep the warps of all rays
-// in flight at once, 6 per SM (plan_lanes has the reasons and the 2-D figures).
-inline int lanes3(long long njobs, int sm_count)
+// Rays per warp of a 3-D or Nx2D trace: as few as keep the warps of all rays in
+// flight at once, 6 per SM (plan_lanes has the reasons and the 2-D figures), or 1
+// per SM where the launch takes the general step (walk false: a batch of hexahedral
+// and 1-D oceans), whose code outgrows the instruction caches, so that warps delay
+// one another. 6 and 1 per SM, and 32 rays a warp in brackets: 558 rays 5.5 and 5.1
+// ms (6.3), 4514 rays 9.8 and 5.8 (5.9), 10010 rays 11.8 and 8.8 (8.7).
+inline int lanes3(long long njobs, int sm_count, bool walk)
 {
+    const long long warps = (walk ? 6LL : 1LL) * sm_count;
     int l = 1;
-    while(l < 32 && (njobs + l - 1) / l > 6LL * sm_count) l *= 2;
+    while(l < 32 && (njobs + l - 1) / l > warps) l *= 2;
     return l;
 }
 
