@@ -196,6 +196,11 @@ class Linear:
     def refresh(self):
         self.ops.to_bf16(self.w, self.wb)
 
+    @property
+    def wt(self):
+        """bf16 W^T [n_in][n_out], a copy: the products read W itself."""
+        return self.ops.T(self.wb)
+
     def params(self):
         return self.w.numel() + self.b.numel()
 
