@@ -161,6 +161,9 @@ __device__ __forceinline__ double sqrt_rn(double a)
     return fma(fma(-g, g, a), h, g);
 }
 
+// sqrt(a) of any a; the square of a spreading that has grown without bound is infinite
+__device__ __forceinline__ double sqrt_any(double a) { return a > 1.0e-270 && a < 1.0e270 ? sqrt_rn(a) : sqrt(a); }
+
 // |nextafter(v, 0) - v| of a finite v: the bit pattern below v's magnitude
 __device__ __forceinline__ double spacing_d(double v)
 {

@@ -38,9 +38,6 @@ inline int lanes3(long long njobs, int sm_count, bool walk)
     return l;
 }
 
-// sqrt(a) for a >= 0
-__device__ __forceinline__ double sqrt_any(double a) { return a > 1.0e-280 ? sqrt_rn(a) : sqrt(a); }
-
 // Sound speed at a point: value, gradient, depth curvature, and the
 // reciprocals of c and c^2 for quotients.
 struct Prof3 {

@@ -19,6 +19,7 @@ __global__ void apply(int op, const double *a, const double *b, double *out, int
     case 5: r = x / y; break;
     case 6: r = sqrt(x); break;
     case 7: r = bhcb::rcp_rn(y); break;
+    case 8: r = bhcb::sqrt_any(x); break;
     }
     out[i] = r;
 }

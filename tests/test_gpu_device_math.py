@@ -126,3 +126,5 @@ def test_roots(device):
     ones = np.array(mantissas(random.Random(8), 100000), np.float64)
     x = np.concatenate([a, scaled(g, np.concatenate([ones, g.uniform(1.0, 4.0, 1000000)]), 420), [2.0 ** -900, 2.0 ** 900]])
     assert same(device(4, x, x), np.sqrt(x)) and same(device(6, x, x), np.sqrt(x))
+    ends = np.array([0.0, 5e-324, 1e-310, 1e-300, 1e-280, 1e-270, 1e270, 1e280, 1.7e308, np.inf])
+    assert same(device(8, ends, ends), np.sqrt(ends)) and same(device(8, x, x), np.sqrt(x))
