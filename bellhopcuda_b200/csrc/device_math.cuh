@@ -132,7 +132,9 @@ __device__ __forceinline__ double rcp_rn(double b)
     return fma(y, e, y);
 }
 __device__ __forceinline__ double rcp_signed(double b) { return copysign(rcp_rn(fabs(b)), b); }
-// 1 / bsq, bsq = b * b rounded and y = rcp_rn(b)
+// 1 / bsq, bsq = b * b rounded and y = rcp_rn(b). y * y is up to two ulps off, after
+// which one step alone misses six mantissas of b (those whose bsq times an odd 54-bit
+// integer is next to a power of two).
 __device__ __forceinline__ double rcp_square(double bsq, double y)
 {
     double z = y * y;

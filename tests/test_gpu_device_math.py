@@ -97,7 +97,10 @@ def test_divisors(device):
     assert same(device(7, wide, np.abs(wide)), 1.0 / np.abs(wide))
     not_ones = wide[(wide > 0.0) | (wide.view(np.int64) & ((1 << 52) - 1) != (1 << 52) - 1)]
     assert same(device(7, not_ones, not_ones), 1.0 / not_ones)
-    half = np.concatenate([scaled(g, b, 440), [2.0 ** 449, 2.0 ** -449, 1500.0]])
+    # the six b whose squares' reciprocals lie so near a midpoint that one Newton step misses it
+    six = np.array([0x17e23ea0c37857, 0x18da7d634a84b0, 0x1f0cba276f78fb, 0x108360cd3ed557, 0x175a6a5d5f9e1e,
+                    0x1aac5548dbdf1c], np.float64) * 2.0 ** -52
+    half = np.concatenate([scaled(g, b, 440), [2.0 ** 449, 2.0 ** -449, 1500.0], six, 1024.0 * six])
     assert same(device(2, half, half), 1.0 / (half * half))
     assert same(device(5, np.ones_like(wide), wide), 1.0 / wide)
 
