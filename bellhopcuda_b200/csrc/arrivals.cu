@@ -178,7 +178,8 @@ __global__ void rs_hist_kernel(const uint64_t *__restrict__ keys, unsigned long 
 
 // One block per digit: exclusive scan of its ntiles counts; its total goes to
 // hist[256 ntiles + digit], and the scatter adds the digits before it. One block
-// of 1024 threads over all digits took 650 us for 1553 tiles, this 6.
+// of 1024 threads over all digits took 650 us for 6.4 M keys (1553 tiles of 4096),
+// this 8 us for 6.0 M (5827 tiles of 1024).
 __global__ void __launch_bounds__(256) rs_scan_kernel(uint32_t *hist, int ntiles)
 {
     __shared__ uint32_t part[8];
