@@ -166,6 +166,16 @@ __device__ __forceinline__ double sqrt_rn(double a)
 // sqrt(a) of any a; the square of a spreading that has grown without bound is infinite
 __device__ __forceinline__ double sqrt_any(double a) { return a > 1.0e-270 && a < 1.0e270 ? sqrt_rn(a) : sqrt(a); }
 
+// The exponents of a ray's p (2^961 or more) or q (infinite, NaN) are so large that the
+// terms 0 q of an ocean without depth curvature, nothing in all other steps, are not
+// numbers. p and q are of the step's start; q at half the step, q + h c p, can only
+// overflow with such a p.
+__device__ __forceinline__ int exponent_bits(double v) { return __double2hiint(v) & 0x7fffffff; }
+__device__ __forceinline__ bool past_numbers(int p_bits, int q_bits)
+{
+    return p_bits >= 0x7c000000 || q_bits >= 0x7ff00000;
+}
+
 // |nextafter(v, 0) - v| of a finite v: the bit pattern below v's magnitude
 __device__ __forceinline__ double spacing_d(double v)
 {

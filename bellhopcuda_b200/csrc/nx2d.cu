@@ -414,6 +414,8 @@ template<bool HEX> struct RayNWalk {
         w.begin();
         double h = w.deltas, halfh = 0.0, w0 = 0.0, w1 = 0.0, cnn1 = 0.0;
         V2<double> u = u0, pm = p0.p, qm = p0.q, gb = ga;
+        const bool past = HEX && past_numbers(max(exponent_bits(p0.p.x), exponent_bits(p0.p.y)),
+                                              max(exponent_bits(p0.q.x), exponent_bits(p0.q.y)));
         Prof3 b = a;
         // one copy of the crossing tests and of the evaluation (Ray3Walk::step)
 #pragma unroll 1
@@ -448,7 +450,8 @@ template<bool HEX> struct RayNWalk {
                 r2.taur = p0.taur + d0.r + d1.r;
                 r2.taui = p0.taui + d0.i + d1.i;
                 const V2<double> pq1p = scl2(-cnn1, qm), pq1q = scl2(b.c, pm);
-                r2.p = HEX ? pm : add2(add2(p0.p, scl2(k, pq0p)), scl2(hw1, pq1p));
+                if(HEX) r2.p = past ? add2(pm, scl2(0.0, qm)) : p0.p;
+                else r2.p = add2(add2(p0.p, scl2(k, pq0p)), scl2(hw1, pq1p));
                 r2.q = add2(add2(p0.q, scl2(k, pq0q)), scl2(hw1, pq1q));
                 r2.x = x;
                 r2.t = t;
@@ -463,7 +466,8 @@ template<bool HEX> struct RayNWalk {
             gb = grad(o);
             cnn1 = o.czz * t.x * t.x;
             // HEX: czz is 0, and p changes by 0 q only (Ray2Seg::step)
-            pm = HEX ? mk2(fma(0.0, p0.q.x, p0.p.x), fma(0.0, p0.q.y, p0.p.y)) : add2(p0.p, scl2(halfh, pq0p));
+            if(!HEX) pm = add2(p0.p, scl2(halfh, pq0p));
+            else if(past) pm = add2(p0.p, scl2(0.0, p0.q));
             qm = add2(p0.q, scl2(halfh, pq0q));
             u = scl2(o.c, t);
         }

@@ -119,3 +119,47 @@ def test_nx2d_step_past_all_numbers(tmp_path):
     b = write_files({".env": flat}, os.path.join(str(tmp_path), "b"))
     (sa, ea), (sb, eb) = evals([a]), evals([b])
     assert evals([a, b]) == (sa + sb, ea + eb)
+
+
+def trap():
+    """A horizontal ray along an interface of a hexahedral ocean: it is caught in small
+    steps, and its p is 5e304 when the half step, whose length is still the full one,
+    takes q past all numbers."""
+    x, y = np.linspace(-20.8, 20.8, 2), np.linspace(-20.8, 20.8, 5)
+    bty = np.array([[2708.02, 3189.64, 3012.39, 2980.44, 2837.09], [2577.44, 3844.82, 3221.02, 3408.98, 2474.34]])
+    ati = np.array([[65.89, 132.56, 14.16, 111.71, 165.63], [146.13, 23.79, 68.95, 113.63, 67.39]])
+    z = np.array([0.0, 2000.0, 4000.0])
+    c = [1492.1967, 1497.4665, 1494.9830, 1492.4996, 1497.7694, 1491.8159, 1497.0857, 1494.6023, 1492.1188, 1497.3886,
+         1494.9378, 1500.2077, 1497.7242, 1495.2407, 1500.5106, 1491.8159, 1497.0857, 1494.6023, 1492.1188, 1497.3886,
+         1492.1967, 1497.4665, 1494.9830, 1492.4996, 1497.7694, 1492.1039, 1497.3737, 1494.8902, 1492.4068, 1497.6766,
+         1491.7231, 1496.9929, 1494.5095, 1492.0260, 1497.2958, 1494.8450, 1500.1149, 1497.6314, 1495.1479, 1500.4178,
+         1491.7231, 1496.9929, 1494.5095, 1492.0260, 1497.2958, 1492.1039, 1497.3737, 1494.8902, 1492.4068, 1497.6766,
+         1509.3154, 1514.5853, 1512.1018, 1509.6183, 1514.8882, 1508.9346, 1514.2045, 1511.7210, 1509.2375, 1514.5074,
+         1512.0566, 1517.3265, 1514.8430, 1512.3595, 1517.6294, 1508.9346, 1514.2045, 1511.7210, 1509.2375, 1514.5074,
+         1509.3154, 1514.5853, 1512.1018, 1509.6183, 1514.8882]
+    env = env_text(title="trap", freq=30.0, ssp_opt="HVW ~", depth=4000.0, ssp=[(0.0, 1495.72), (2000.0, 1495.63),
+                   (4000.0, 1512.84)], bot=("A~", 1650.0, 1.6, 0.5), sx=[-0.3], sy=[-0.25], sz=[2000.0],
+                   rz=[651.57, 838.87, 1858.87, 1996.95, 2487.69, 2955.4, 3655.58], rr_km=[0.0319, 0.2021, 0.2545],
+                   theta=[90.0], run_type="CB   3", alpha=(3, -60.0, 60.0), beta=(9, -30.0, 40.0), step=1333.33,
+                   box_km=(16.8, 12.8), box_z=3200.0)
+    # the file holds one record of x values per (z, y)
+    c = np.array(c).reshape(3, 5, 5).transpose(2, 1, 0)
+    return {".env": env, ".bty": grid_text(x, y, bty, "R"), ".ati": grid_text(x, y, ati, "R"),
+            ".ssp": hex_ssp_text(y, y, z, c)}
+
+
+def test_half_step_past_all_numbers(tmp_path):
+    """As test_nx2d_step_past_all_numbers, in 3-D, for q at the half step."""
+    def evals(roots):
+        with B.Tracer(precision=B.PREC_FP64) as t:
+            for r in roots:
+                t.add_env3d(r)
+            t.run()
+            return t.stats()["steps"], t.stats()["evals"]
+    flat = env_text(title="flat", freq=100.0, ssp_opt="CVW", depth=1000.0, ssp=[(0.0, 1500.0), (1000.0, 1510.0)],
+                    bot=("R",), sx=[0.0], sy=[0.0], sz=[250.0], rz=[300.0], rr_km=[3.0], theta=[0.0], run_type="CB   3",
+                    alpha=(3, -20.0, 20.0), beta=(4, 0.0, 360.0), step=100.0, box_km=(4.2, 4.2), box_z=1100.0)
+    a = write_files(trap(), os.path.join(str(tmp_path), "a"))
+    b = write_files({".env": flat}, os.path.join(str(tmp_path), "b"))
+    (sa, ea), (sb, eb) = evals([a]), evals([b])
+    assert evals([a, b]) == (sa + sb, ea + eb) and sa > 100000
