@@ -173,20 +173,11 @@ template<bool HEX> struct Ray3Walk {
     static __device__ __forceinline__ bool past3(const Ray3 &r)
     {
         const double(&p)[2][2] = r.p.m, (&q)[2][2] = r.q.m;
-        return past_numbers(max(max(exponent_bits(p[0][0]), exponent_bits(p[0][1])),
-                                max(exponent_bits(p[1][0]), exponent_bits(p[1][1]))),
-                            max(max(exponent_bits(q[0][0]), exponent_bits(q[0][1])),
-                                max(exponent_bits(q[1][0]), exponent_bits(q[1][1]))));
-    }
-    // p + q C^T for C = 0
-    static __device__ __forceinline__ M2 zero_q(M2 p, const M2 &q)
-    {
-        for(int i = 0; i < 2; ++i) {
-            const double z = 0.0 * q.m[0][i] + 0.0 * q.m[1][i];
-            p.m[0][i] += z;
-            p.m[1][i] += z;
-        }
-        return p;
+        const int a = exponent_bits(p[0][0]), b = exponent_bits(p[0][1]), c = exponent_bits(p[1][0]);
+        const int d = exponent_bits(p[1][1]);
+        return past_numbers(max(max(a, b), max(c, d)), max(max(exponent_bits(q[0][0]), exponent_bits(q[0][1])),
+                                                           max(exponent_bits(q[1][0]), exponent_bits(q[1][1]))))
+            && min(min(a, b), min(c, d)) <= 0x7ff00000;
     }
     // delta_pq3: rate of the ray normals' angle (horizontal gradients only),
     // p' (with a depth curvature only); q' is c p
@@ -215,7 +206,10 @@ template<bool HEX> struct Ray3Walk {
         const Prof3 a = o0;
         w.begin();
         const bool steep = !(t0.x * t0.x + t0.y * t0.y > 1.0e-200);
-        if(steep) {   // no horizontal direction: the general step
+        // without a curvature p changes by 0 q only (Ray2Seg::step), which matters while p
+        // is a number and p or q is past all numbers
+        const bool past = (HEX || !bent) && past3(p0);
+        if(steep || past) {   // no horizontal direction, or such a p or q: the general step
             Step3IO io;
             io.top = w.general(w.top, w.E->btop, w.E->top_ny);
             io.bot = w.general(w.bot, w.E->bbot, w.E->bot_ny);
@@ -243,10 +237,6 @@ template<bool HEX> struct Ray3Walk {
             const bool curved = !HEX && bent;
             M2 dp0, dp1;
             if(curved) dp0 = p_rate(p0, a);
-            // without a curvature p changes by 0 q only (Ray2Seg::step)
-            const bool past = !curved && past3(p0);
-            M2 ps = p0.p;
-            if(past) ps = zero_q(p0.p, p0.q);
             const V3 u0 = scl3(c0, t0);
             const M2 dq0 = m2_scl(c0, p0.p);
             // Three passes over one copy of the crossing tests and of the
@@ -296,8 +286,7 @@ template<bool HEX> struct Ray3Walk {
                     r2.taui = p0.taui + d0.i + d1.i;
                     r2.phi = (p0.phi + k * f0) + hw1 * f1;
                     const M2 dq1 = m2_scl(b.c, r1.p);
-                    r2.p = curved ? m2_add(m2_add(p0.p, m2_scl(k, dp0)), m2_scl(hw1, dp1)) : ps;
-                    if(past) r2.p = zero_q(r2.p, r1.q);
+                    r2.p = curved ? m2_add(m2_add(p0.p, m2_scl(k, dp0)), m2_scl(hw1, dp1)) : p0.p;
                     r2.q = m2_add(m2_add(p0.q, m2_scl(k, dq0)), m2_scl(hw1, dq1));
                     r2.x = x;
                     r2.t = t;
@@ -312,8 +301,8 @@ template<bool HEX> struct Ray3Walk {
                 r1.x = x;
                 r1.t = t;
                 r1.phi = p0.phi + halfh * f0;
-                r1.p = curved ? m2_add(p0.p, m2_scl(halfh, dp0)) : ps;
-                if(curved || past) r1.q = m2_add(p0.q, m2_scl(halfh, dq0));
+                r1.p = curved ? m2_add(p0.p, m2_scl(halfh, dp0)) : p0.p;
+                if(curved) r1.q = m2_add(p0.q, m2_scl(halfh, dq0));
                 f1 = phi_rate(t, o);
                 if(curved) dp1 = p_rate(r1, o);
                 u = scl3(o.c, t);
