@@ -282,18 +282,15 @@ template<int K> struct Ray2Seg {
         const double c0 = c, g0 = g, csq0 = csq, rc0 = rc, rcsq0 = rcsq;
         // c-linear: czz is 0 and the paraxial p does not change within the step, but by
         // 0 q, which is not a number once q, here or at half the step, has grown past all
-        // numbers
-        const bool past = K == SSP_CLINEAR
-            && past_numbers(max(exponent_bits(p0.p.x), exponent_bits(p0.p.y)),
-                            max(exponent_bits(p0.q.x), exponent_bits(p0.q.y)));
+        // numbers (a test for that costs 2 % of the trace, the multiplications nothing)
         const double cnn0 = czz * t0.x * t0.x;
         const V2<double> pq0p = scl2(-cnn0, p0.q), pq0q = scl2(c0, p0.p);
         const V2<double> u0 = scl2(c0, t0);
         double h = reduce(u0, deltas, za, zb, s0, ctr);
         const double halfh = 0.5 * h, h2 = 2.0 * halfh;
         const V2<double> t1 = mk2(t0.x, t0.y - quot_rn(halfh * g0, csq0, rcsq0));
-        V2<double> pm = K == SSP_CLINEAR ? p0.p : add2(p0.p, scl2(halfh, pq0p));
-        if(past) pm = add2(pm, scl2(0.0, p0.q));
+        const V2<double> pm = K == SSP_CLINEAR ? mk2(fma(0.0, p0.q.x, p0.p.x), fma(0.0, p0.q.y, p0.p.y))
+                                               : add2(p0.p, scl2(halfh, pq0p));
         const V2<double> qm = add2(p0.q, scl2(halfh, pq0q));
         double c1, g1, czz1;
         eval(x0.y + halfh * u0.y, t1.y, c1, g1, czz1);
@@ -341,8 +338,8 @@ template<int K> struct Ray2Seg {
         p1.t = mk2(t0.x, (t0.y - quot_rn(hw0 * g0, csq0, rcsq0)) - quot_rn(hw1 * g1, csq1, rcsq1));
         p1.taur = p0.taur + quot_rn(hw0, c0, rc0) + quot_rn(hw1, c1, rc1);
         p1.taui = p0.taui;
-        p1.p = K == SSP_CLINEAR ? pm : add2(add2(p0.p, scl2(hw0, pq0p)), scl2(hw1, pq1p));
-        if(past) p1.p = add2(p1.p, scl2(0.0, qm));
+        p1.p = K == SSP_CLINEAR ? mk2(fma(0.0, qm.x, pm.x), fma(0.0, qm.y, pm.y))
+                                : add2(add2(p0.p, scl2(hw0, pq0p)), scl2(hw1, pq1p));
         p1.q = add2(add2(p0.q, scl2(hw0, pq0q)), scl2(hw1, pq1q));
         p1.Amp = p0.Amp;
         p1.Phase = p0.Phase;
